@@ -197,7 +197,8 @@ int nb_selftest_bounded_wait(int32_t device, int32_t wait_ms);
  * such knob; LinearBVH::maxLeafSize, LinearBVH.h:135-137, is the one it has): block_threads
  * threads per block (128 or 256) and slab_entries staged partially accepted nodes per warp (32 or
  * 64); 0 selects the default (256, 64). Decisions and interaction counts do not depend on it;
- * accelerations sum the same terms, possibly in another order. The autotuner
+ * accelerations sum the same terms, possibly in another order. Passes over few bodies, which run one
+ * block per 32 targets, keep their own block size (same results). The autotuner
  * (nbody_b200/autotune.py) picks it per workload. */
 int nb_set_traversal_shape(nb_ctx *ctx, int32_t block_threads, int32_t slab_entries);
 int nb_get_traversal_shape(const nb_ctx *ctx, int32_t *block_threads, int32_t *slab_entries);

@@ -482,8 +482,8 @@ int force_pass_batch(nb_ctx *ctx, Marks &mk) {
     ctx->sorted_codes = ctx->sw.keys_alt;
     mk.mark(kTraverse);
     cudaMemsetAsync(ctx->inst_counts, 0, (size_t) 2 * ctx->num_inst * sizeof(unsigned long long), s);
-    launch_bh_traverse(ctx->cfg.order, ctx->nodes, ctx->tw.num_nodes, ctx->pos, n, ctx->pos, n, ctx->cfg.G,
-                       ctx->cfg.epsilon, ctx->acc, ctx->counts, ctx->trav, ctx->err, s, ctx->groups, ctx->ngroups,
+    launch_bh_traverse(ctx->cfg.order, ctx->nodes, ctx->tw.num_nodes, ctx->pos, n, ctx->pos, n,
+                       ctx->cfg.max_leaf_size, ctx->cfg.G, ctx->cfg.epsilon, ctx->acc, ctx->counts, ctx->trav, ctx->err, s, ctx->groups, ctx->ngroups,
                        ctx->inst_root, ctx->inst_counts);
     ctx->have_tree = true;
     ctx->acc_is_bh = true;
@@ -544,7 +544,7 @@ int force_pass(nb_ctx *ctx, Marks &mk) {
     mk.mark(kTraverse);
     // a sharded context evaluates only its slice of the Morton-ordered targets
     launch_bh_traverse(ctx->cfg.order, ctx->nodes, ctx->tw.num_nodes, ctx->pos, n, ctx->pos + first, count,
-                       ctx->cfg.G, ctx->cfg.epsilon, ctx->acc + first, ctx->counts, ctx->trav, ctx->err, s);
+                       ctx->cfg.max_leaf_size, ctx->cfg.G, ctx->cfg.epsilon, ctx->acc + first, ctx->counts, ctx->trav, ctx->err, s);
     ctx->have_tree = true;
     ctx->acc_is_bh = true;
     if (ctx->timing) ctx->times.launches += launches_per_pass(ctx, need_bbox, false);
@@ -624,7 +624,7 @@ int nb_create(const nb_config *cfg, nb_ctx **out) {
         return NB_ERR_OUT_OF_MEMORY;
     }
     ctx->trav.warps = traverse_resident_warps(cfg->device);
-    if (dev_alloc(&ctx->trav.stack, (size_t) ctx->trav.warps * kTraverseStack) != cudaSuccess ||
+    if (dev_alloc(&ctx->trav.stack, (size_t) ctx->trav.warps * kWarpScratch) != cudaSuccess ||
         dev_alloc(&ctx->trav.group_counter, 1) != cudaSuccess) {
         nb_destroy(ctx);
         return NB_ERR_OUT_OF_MEMORY;

@@ -295,7 +295,8 @@ void launch_dual_traverse(const DualNodes &nodes, const int *num_nodes, const fl
 
 // traverse.cu
 struct TraverseWorkspace {
-    int2 *stack = nullptr;            // per resident warp: kTraverseStack entries of (node, target mask)
+    int2 *stack = nullptr;            // per resident warp: kTraverseStack entries of (node, target mask), then
+                                      // the warp's leaf sums (kWarpScratch int2 in all)
     unsigned *group_counter = nullptr;
     int64_t warps = 0;                // resident warps the stack memory was sized for
     int threads = 256;                // launch shape: threads per block (128 or 256)
@@ -304,14 +305,16 @@ struct TraverseWorkspace {
 // Whether (threads, slab) is one of the traversal's compiled launch shapes.
 bool traversal_shape_valid(int threads, int slab);
 constexpr int kTraverseStack = 4608;
+constexpr int kWarpScratch = kTraverseStack + 288;  // int2 per resident warp: the stack, then its leaf sums
 // Resident warps of the persistent traversal grid on `device` (for sizing TraverseWorkspace).
 int64_t traverse_resident_warps(int device);
 // groups (optional): one int4 (first target, target count <= 32, instance, 0) per warp task; the
 // traversal of a group starts at inst_root[instance]. Without groups, targets are cut into
 // consecutive groups of 32 that start at node 0. inst_counts (optional, with groups): per instance,
-// (particle-particle, node-particle) interaction counts are added at [2 * instance + {0, 1}].
+// (particle-particle, node-particle) interaction counts are added at [2 * instance + {0, 1}]. leaf:
+// the tree's largest leaf (it moves the line between the traversal's two forms, nothing else).
 void launch_bh_traverse(int order, const NodeArrays &nodes, const int *num_nodes, const float4 *bodies, int64_t n_bodies,
-                        const float4 *targets, int64_t n_targets, float G, float eps, float4 *acc,
+                        const float4 *targets, int64_t n_targets, int leaf, float G, float eps, float4 *acc,
                         unsigned long long *counts, TraverseWorkspace &ws, uint32_t *err, cudaStream_t s,
                         const int4 *groups = nullptr, int64_t num_groups = 0, const int *inst_root = nullptr,
                         unsigned long long *inst_counts = nullptr);

@@ -23,12 +23,15 @@
 //      32 targets (broadcast from shared memory), producing accept and open masks.
 //   3. Accepted nodes are staged in per-warp shared-memory slabs: the lane that accepted a node
 //      copies its payload there asynchronously (cp.async), so the payload crosses L2 once per
-//      group instead of once per target. Nodes accepted by every target go to the full slab and
-//      are evaluated by all lanes with broadcast reads; nodes accepted by some targets go to the
-//      partial slab with their target masks, and at evaluation a warp bit-matrix transpose of
-//      the masks gives every lane the set of slab entries it owns, which it walks on its own.
-//      Opened leaves go to a (leaf, mask) list evaluated with broadcast body loads; opened
-//      internal nodes push both children.
+//      group instead of once per target. Nodes accepted by every target go to the full slab, are
+//      rewritten there as pair records and evaluated by all lanes with broadcast reads, two nodes per
+//      paired FP32 instruction; nodes accepted by some targets go to the partial slab with their
+//      target masks, and at evaluation a warp bit-matrix transpose of the masks gives every lane the
+//      set of slab entries it owns, which it walks on its own. Opened leaves go to a (leaf, mask)
+//      list, whose bodies are packed into shared-memory tiles of 32 and evaluated two per instruction;
+//      opened internal nodes push both children.
+//   4. Launches of few groups run the same walk with a team of eight warps per group
+//      (bh_team_kernel): the walker hands its slabs and lists to the other warps.
 //
 // Arithmetic: FP32, one MUFU rsqrt per interaction, G applied once per target. Pair term:
 // 20 flops by the usual direct-sum convention (12 FP32 instructions + rsqrt). Quadrupole node
@@ -63,6 +66,9 @@ struct WarpSmem {
     float4 full_pay[kFullSlab * PAY];  // payloads of group-wide accepted nodes
     float4 part_pay[(PART + 1) * PAY]; // payloads of partially accepted nodes, then the null payload
     uint32_t part_mask[PART];          // their target masks
+    unsigned node_count[32], pair_count[32];  // the group's interactions per target
+    int turn;                          // leaf set of the next list
+    int pad[3];
     int pp_begin[kList], pp_end[kList];
     uint32_t pp_mask[kList];
     int mixed_node[kList];
@@ -161,37 +167,181 @@ __device__ __forceinline__ void stage_node(float4 *dst, const float4 *__restrict
     for (int k = 0; k < PAY; ++k) cp_async16(dst + k, src + k);
 }
 
-// Nodes accepted by the whole group: every lane evaluates every staged entry (broadcast reads).
-template<int ORDER, bool EPS0, int PART>
-__device__ __forceinline__ void flush_full(WarpSmem<NodeLayout<ORDER>::PAY, PART> &S, int &nfull, float4 p, float eps,
-                                           float &ax, float &ay, float &az, unsigned &cnp) {
-    constexpr int PAY = NodeLayout<ORDER>::PAY;
-    cp_async_wait_all();
-    __syncwarp();
-    int j = 0;
-    for (; j + 1 < nfull; j += 2) {
-        staged_term<ORDER, EPS0>(S.full_pay + j * PAY, p, eps, ax, ay, az);
-        staged_term<ORDER, EPS0>(S.full_pay + (j + 1) * PAY, p, eps, ax, ay, az);
-    }
-    if (j < nfull) staged_term<ORDER, EPS0>(S.full_pay + j * PAY, p, eps, ax, ay, az);
-    cnp += (unsigned) nfull;
-    nfull = 0;
-    __syncwarp();
+// A target's sums are kept apart as one set for the approximated nodes and kLeafSets sets for the
+// pairs of opened leaves (the q-th flushed list goes to set q % kLeafSets), each in the order of the
+// flushed slabs and lists, and added at the end in set order. A set's terms and their order depend
+// on the walk alone, so one warp (bh_kernel) and a team of warps that share the sets
+// (bh_team_kernel) give the same bits.
+constexpr int kLeafSets = 6;
+constexpr int kLeafFlush = 32;  // a list of more leaves than this is flushed at the end of the round
+static_assert(kLeafFlush + 32 <= kList, "a round appends at most 32 leaves");
+
+// pair2_term with each body's factor set to zero where `on` is false.
+template<bool EPS0>
+__device__ __forceinline__ void masked_pair2(float2 npx, float2 npy, float2 npz, float2 eps2, float4 u, float4 v,
+                                             bool on_a, bool on_b, float2 &ax, float2 &ay, float2 &az) {
+    const float2 dx = __fadd2_rn(make_float2(u.x, u.y), npx);
+    const float2 dy = __fadd2_rn(make_float2(u.z, u.w), npy);
+    const float2 dz = __fadd2_rn(make_float2(v.x, v.y), npz);
+    const float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __ffma2_rn(dz, dz, eps2)));
+    float2 inv;
+    inv.x = rsqrt_hw(r2.x);
+    inv.y = rsqrt_hw(r2.y);
+    float2 s = __fmul2_rn(make_float2(v.z, v.w), __fmul2_rn(__fmul2_rn(inv, inv), inv));
+    s.x = on_a && !(EPS0 && r2.x == 0.f) ? s.x : 0.f;
+    s.y = on_b && !(EPS0 && r2.y == 0.f) ? s.y : 0.f;
+    ax = __ffma2_rn(dx, s, ax);
+    ay = __ffma2_rn(dy, s, ay);
+    az = __ffma2_rn(dz, s, az);
 }
 
-// Nodes accepted by some targets only: the masks are transposed so that each lane holds the set
-// of entries it evaluates, then every lane walks its own set.
-template<int ORDER, bool EPS0, int PART>
-__device__ __forceinline__ void flush_part(WarpSmem<NodeLayout<ORDER>::PAY, PART> &S, int &npart, float4 p, float eps,
-                                           int lane, float &ax, float &ay, float &az, unsigned &cnp) {
+// Two quadrupole node terms at once in paired FP32 arithmetic, operand pairs as in pair2_term:
+// u = (x_a, x_b, y_a, y_b), v = (z_a, z_b, M_a, M_b), then the moments Qxx, Qxy | Qxz, Qyy | Qyz, Qzz | 1.5 tr Q
+// of both nodes. With d = com - p the terms of quad_term change sign in both factors.
+template<bool EPS0>
+__device__ __forceinline__ void quad2_term(float2 npx, float2 npy, float2 npz, float2 eps2, const float4 *rec,
+                                           float2 &ax, float2 &ay, float2 &az) {
+    const float4 u = rec[0], v = rec[1], q0 = rec[2], q1 = rec[3], q2 = rec[4];
+    const float2 tr = *reinterpret_cast<const float2 *>(rec + 5);
+    const float2 dx = __fadd2_rn(make_float2(u.x, u.y), npx);
+    const float2 dy = __fadd2_rn(make_float2(u.z, u.w), npy);
+    const float2 dz = __fadd2_rn(make_float2(v.x, v.y), npz);
+    const float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __ffma2_rn(dz, dz, eps2)));
+    float2 inv;
+    inv.x = rsqrt_hw(r2.x);
+    inv.y = rsqrt_hw(r2.y);
+    if (EPS0) {
+        if (r2.x == 0.f) inv.x = 0.f;
+        if (r2.y == 0.f) inv.y = 0.f;
+    }
+    const float2 inv2 = __fmul2_rn(inv, inv), inv3 = __fmul2_rn(inv2, inv);
+    const float2 inv5 = __fmul2_rn(inv3, inv2), inv7 = __fmul2_rn(inv5, inv2);
+    const float2 xx = make_float2(q0.x, q0.y), xy = make_float2(q0.z, q0.w), xz = make_float2(q1.x, q1.y);
+    const float2 yy = make_float2(q1.z, q1.w), yz = make_float2(q2.x, q2.y), zz = make_float2(q2.z, q2.w);
+    const float2 qx = __ffma2_rn(xx, dx, __ffma2_rn(xy, dy, __fmul2_rn(xz, dz)));
+    const float2 qy = __ffma2_rn(xy, dx, __ffma2_rn(yy, dy, __fmul2_rn(yz, dz)));
+    const float2 qz = __ffma2_rn(xz, dx, __ffma2_rn(yz, dy, __fmul2_rn(zz, dz)));
+    const float2 dqd = __ffma2_rn(dx, qx, __ffma2_rn(dy, qy, __fmul2_rn(dz, qz)));
+    const float2 mono = __fmul2_rn(make_float2(v.z, v.w), inv3);
+    const float2 sr = __ffma2_rn(__fmul2_rn(make_float2(7.5f, 7.5f), inv7), dqd,
+                                 __ffma2_rn(make_float2(-tr.x, -tr.y), inv5, mono));
+    const float2 sq = __fmul2_rn(make_float2(-3.0f, -3.0f), inv5);
+    ax = __ffma2_rn(dx, sr, __ffma2_rn(qx, sq, ax));
+    ay = __ffma2_rn(dy, sr, __ffma2_rn(qy, sq, ay));
+    az = __ffma2_rn(dz, sr, __ffma2_rn(qz, sq, az));
+}
+
+// Staged nodes accepted by the whole group (n <= 32, one payload per slot): the slots are rewritten
+// as pair records in place, a null payload filling an odd last one, and every lane evaluates every
+// pair (broadcast reads).
+template<int ORDER, bool EPS0>
+__device__ __forceinline__ void full_terms(float4 *pay, int n, float4 p, float eps, int lane, float &ax, float &ay,
+                                           float &az) {
     constexpr int PAY = NodeLayout<ORDER>::PAY;
-    cp_async_wait_all();
+    float4 c[PAY];
+#pragma unroll
+    for (int k = 0; k < PAY; ++k) c[k] = k == 0 ? make_float4(1e30f, 1e30f, 1e30f, 0.f) : make_float4(0.f, 0.f, 0.f, 0.f);
+    if (lane < n) {
+#pragma unroll
+        for (int k = 0; k < PAY; ++k) c[k] = pay[lane * PAY + k];
+    }
     __syncwarp();
-    uint32_t b0 = transpose32(lane < npart ? S.part_mask[lane] : 0u, lane);
+    if (lane <= n && lane < 32) {
+        float *rec = reinterpret_cast<float *>(pay + (lane & ~1) * PAY) + (lane & 1);
+#pragma unroll
+        for (int k = 0; k < PAY; ++k) {
+            rec[8 * k] = c[k].x;
+            rec[8 * k + 2] = c[k].y;
+            rec[8 * k + 4] = c[k].z;
+            rec[8 * k + 6] = c[k].w;
+        }
+    }
+    __syncwarp();
+    const float2 npx = make_float2(-p.x, -p.x), npy = make_float2(-p.y, -p.y), npz = make_float2(-p.z, -p.z);
+    const float2 eps2 = make_float2(eps, eps);
+    float2 sx = make_float2(ax, 0.f), sy = make_float2(ay, 0.f), sz = make_float2(az, 0.f);
+    for (int j = 0; j < n; j += 2) {
+        const float4 *rec = pay + j * PAY;
+        if constexpr (ORDER == 1) pair2_term<EPS0>(npx, npy, npz, eps2, rec[0], rec[1], sx, sy, sz);
+        else quad2_term<EPS0>(npx, npy, npz, eps2, rec, sx, sy, sz);
+    }
+    ax = sx.x + sx.y;
+    ay = sy.x + sy.y;
+    az = sz.x + sz.y;
+}
+
+// The bodies of a list of opened leaves (n ranges [begin, end) with target masks) for every target.
+// They are packed back to back into tiles of 32, stored as 16 interleaved pairs (two bodies per paired
+// FP32 instruction) in shared memory (512 bytes); the transposed masks tell each lane which bodies of
+// the tile its target takes, and the others' factors are set to zero. A tile's bodies are loaded,
+// one per lane, while the tile before it is evaluated. Returns the lane's number of pairs.
+template<bool EPS0>
+__device__ __forceinline__ unsigned leaf_terms(const int *begin, const int *end, const uint32_t *mask, int n,
+                                               const float4 *__restrict__ bodies, float4 *tile, float4 p, float eps,
+                                               int lane, float &ax, float &ay, float &az) {
+    unsigned pairs = 0;
+    int j = 0, o = n > 0 ? begin[0] : 0, e = n > 0 ? end[0] : 0, fill = 0;
+    float4 body;
+    uint32_t who;
+    auto fetch = [&]() {
+        fill = 0;
+        who = 0u;
+        body = make_float4(0.f, 0.f, 0.f, 0.f);
+        while (j < n) {
+            const int take = min(e - o, 32 - fill);
+            if (lane >= fill && lane < fill + take) {
+                body = __ldg(bodies + o + (lane - fill));
+                who = mask[j];
+            }
+            fill += take;
+            o += take;
+            if (o < e) break;
+            if (++j < n) {
+                o = begin[j];
+                e = end[j];
+            }
+            if (fill == 32) break;
+        }
+    };
+    fetch();
+    const float2 npx = make_float2(-p.x, -p.x), npy = make_float2(-p.y, -p.y), npz = make_float2(-p.z, -p.z);
+    const float2 eps2 = make_float2(eps, eps);
+    float2 sx = make_float2(ax, 0.f), sy = make_float2(ay, 0.f), sz = make_float2(az, 0.f);
+    while (fill > 0) {
+        const int m = fill;
+        uint32_t bits = transpose32(who, lane);
+        pairs += __popc(bits);
+        float *f = reinterpret_cast<float *>(tile) + (lane >> 1) * 8 + (lane & 1);
+        f[0] = body.x;
+        f[2] = body.y;
+        f[4] = body.z;
+        f[6] = body.w;
+        __syncwarp();
+        fetch();
+        for (int b = 0; b < m; b += 4, bits >>= 4) {
+            const float4 u0 = tile[b], v0 = tile[b + 1], u1 = tile[b + 2], v1 = tile[b + 3];
+            masked_pair2<EPS0>(npx, npy, npz, eps2, u0, v0, bits & 1u, bits & 2u, sx, sy, sz);
+            masked_pair2<EPS0>(npx, npy, npz, eps2, u1, v1, bits & 4u, bits & 8u, sx, sy, sz);
+        }
+        __syncwarp();
+    }
+    ax = sx.x + sx.y;
+    ay = sy.x + sy.y;
+    az = sz.x + sz.y;
+    return pairs;
+}
+
+// Staged nodes accepted by some targets only: the masks are transposed so that each lane holds the
+// set of entries it evaluates, then every lane walks its own set. null is the slot of the null payload.
+// Returns the lane's number of entries.
+template<int ORDER, bool EPS0, int PART>
+__device__ __forceinline__ unsigned part_terms(const float4 *pay, const uint32_t *mask, int n, float4 p, float eps,
+                                               int lane, float &ax, float &ay, float &az) {
+    constexpr int PAY = NodeLayout<ORDER>::PAY;
+    uint32_t b0 = transpose32(lane < n ? mask[lane] : 0u, lane);
     uint32_t b1 = 0u;
-    if constexpr (PART > 32)
-        b1 = npart > 32 ? transpose32(lane + 32 < npart ? S.part_mask[lane + 32] : 0u, lane) : 0u;
-    cnp += (unsigned) (__popc(b0) + __popc(b1));
+    if constexpr (PART > 32) b1 = n > 32 ? transpose32(lane + 32 < n ? mask[lane + 32] : 0u, lane) : 0u;
+    const unsigned taken = (unsigned) (__popc(b0) + __popc(b1));
     // a lane whose set is used up evaluates the null payload instead of branching around the term
     while (__any_sync(kFull, (b0 | b1) != 0u)) {
         int j = PART;
@@ -202,78 +352,309 @@ __device__ __forceinline__ void flush_part(WarpSmem<NodeLayout<ORDER>::PAY, PART
             j = 31 + __ffs(b1);
             b1 &= b1 - 1;
         }
-        staged_term<ORDER, EPS0>(S.part_pay + j * PAY, p, eps, ax, ay, az);
+        staged_term<ORDER, EPS0>(pay + j * PAY, p, eps, ax, ay, az);
     }
-    npart = 0;
-    __syncwarp();
+    return taken;
 }
 
-template<bool EPS0, int PAY, int PART>
-__device__ __forceinline__ void flush_pp(WarpSmem<PAY, PART> &S, int &npp, const float4 *__restrict__ bodies, float4 p,
-                                         float eps, int lane, float &ax, float &ay, float &az, unsigned &cpp) {
-    for (int j = 0; j < npp; ++j) {
-        const int b = S.pp_begin[j], e = S.pp_end[j];
-        const bool on = (S.pp_mask[j] >> lane) & 1u;
-        int k = b;
-        for (; k + 3 < e; k += 4) {
-            const float4 s0 = __ldg(bodies + k), s1 = __ldg(bodies + k + 1);
-            const float4 s2 = __ldg(bodies + k + 2), s3 = __ldg(bodies + k + 3);
-            pair_term<EPS0>(p, s0, eps, ax, ay, az, on);
-            pair_term<EPS0>(p, s1, eps, ax, ay, az, on);
-            pair_term<EPS0>(p, s2, eps, ax, ay, az, on);
-            pair_term<EPS0>(p, s3, eps, ax, ay, az, on);
-        }
-        for (; k < e; ++k) {
-            const float4 s0 = __ldg(bodies + k);
-            pair_term<EPS0>(p, s0, eps, ax, ay, az, on);
-        }
-        if (on) cpp += (unsigned) (e - b);
-    }
-    npp = 0;
-    __syncwarp();
+// The null payload: no mass and no moments at 1e30 on every axis, where the squared distance from
+// any target with coordinates below 1e29 in magnitude overflows to infinity, so that every factor of
+// the term is exactly zero and it adds nothing.
+template<int PAY>
+__device__ __forceinline__ void write_null_payload(float4 *slot, int lane) {
+    if (lane < PAY) slot[lane] = lane == 0 ? make_float4(1e30f, 1e30f, 1e30f, 0.f) : make_float4(0.f, 0.f, 0.f, 0.f);
 }
 
-// Classified entries of one round, appended to the slabs and lists (warp-uniform control flow):
-// acc / part are accepted nodes (target mask mk for part), leaf is an opened leaf (body range
-// l0..l1, mask mk), open an opened internal node (children c + 1 and l0, mask mk), mixed a node
-// still to be resolved per target.
+// Where a walk's findings go in bh_kernel: staged in the warp's slabs and evaluated by the warp
+// itself when a slab or list could overflow. The node set is kept in registers; the leaf sets stay
+// in global scratch (L2) and the interaction counts in shared memory between flushes.
 template<int ORDER, bool EPS0, int PART>
-__device__ __forceinline__ bool dispatch(WarpSmem<NodeLayout<ORDER>::PAY, PART> &S, const float4 *__restrict__ pay,
-                                         const float4 *__restrict__ bodies, int2 *stack, bool acc, bool part,
-                                         bool leaf, bool open, bool mixed, int c, uint32_t mk, int l0, int l1,
-                                         int n_bodies, uint32_t lt, int lane, int &nfull, int &npart, int &npp,
-                                         int &nmixed, int &top, float4 p, float eps, float &ax, float &ay, float &az,
-                                         unsigned &gnp, unsigned &gpp, uint32_t *err) {
-    constexpr int PAY = NodeLayout<ORDER>::PAY;
-    uint32_t b = __ballot_sync(kFull, acc);
-    if (b) {
-        if (nfull + __popc(b) > kFullSlab) flush_full<ORDER, EPS0, PART>(S, nfull, p, eps, ax, ay, az, gnp);
-        if (acc) stage_node<PAY>(S.full_pay + (nfull + __popc(b & lt)) * PAY, pay, c);
+struct WarpSink {
+    static constexpr int PAY = NodeLayout<ORDER>::PAY;
+    WarpSmem<PAY, PART> &S;
+    const float4 *__restrict__ pay;
+    const float4 *__restrict__ bodies;
+    float4 p;
+    float eps;
+    int lane, n_bodies;
+    int nfull = 0, npart = 0, npp = 0;
+    float ax = 0.f, ay = 0.f, az = 0.f;  // the node set
+    float *sets;  // kLeafSets x 3 x 32 floats of the warp's global scratch
+
+    __device__ __forceinline__ void clear() {
+        for (int k = 0; k < 3 * kLeafSets; ++k) sets[k * 32 + lane] = 0.f;
+        S.node_count[lane] = S.pair_count[lane] = 0u;
+        if (lane == 0) S.turn = 0;
+    }
+    __device__ __forceinline__ void flush_full() {
+        cp_async_wait_all();
+        __syncwarp();
+        full_terms<ORDER, EPS0>(S.full_pay, nfull, p, eps, lane, ax, ay, az);
+        S.node_count[lane] += (unsigned) nfull;
+        nfull = 0;
+        __syncwarp();
+    }
+    __device__ __forceinline__ void flush_part() {
+        cp_async_wait_all();
+        __syncwarp();
+        S.node_count[lane] += part_terms<ORDER, EPS0, PART>(S.part_pay, S.part_mask, npart, p, eps, lane, ax, ay, az);
+        npart = 0;
+        __syncwarp();
+    }
+    __device__ __forceinline__ void flush_leaves() {
+        if (nfull > 0) flush_full();  // the full slab's memory holds the tiles
+        float *mine = sets + S.turn * 96 + lane;
+        float sx = mine[0], sy = mine[32], sz = mine[64];
+        const unsigned pairs = leaf_terms<EPS0>(S.pp_begin, S.pp_end, S.pp_mask, npp, bodies, S.full_pay, p, eps, lane,
+                                                sx, sy, sz);
+        mine[0] = sx;
+        mine[32] = sy;
+        mine[64] = sz;
+        S.pair_count[lane] += pairs;
+        npp = 0;
+        __syncwarp();
+        if (lane == 0) S.turn = S.turn + 1 < kLeafSets ? S.turn + 1 : 0;
+        __syncwarp();
+    }
+    // accepted by every target / by the targets in mk (b: the ballot of on)
+    __device__ __forceinline__ void add_full(bool on, uint32_t b, uint32_t lt, int c) {
+        if (nfull + __popc(b) > kFullSlab) flush_full();
+        if (on) stage_node<PAY>(S.full_pay + (nfull + __popc(b & lt)) * PAY, pay, c);
         nfull += __popc(b);
     }
-    b = __ballot_sync(kFull, part);
-    if (b) {
-        if (npart + __popc(b) > PART) flush_part<ORDER, EPS0, PART>(S, npart, p, eps, lane, ax, ay, az, gnp);
-        if (part) {
+    __device__ __forceinline__ void add_part(bool on, uint32_t b, uint32_t lt, int c, uint32_t mk) {
+        if (npart + __popc(b) > PART) flush_part();
+        if (on) {
             const int slot = npart + __popc(b & lt);
             stage_node<PAY>(S.part_pay + slot * PAY, pay, c);
             S.part_mask[slot] = mk;
         }
         npart += __popc(b);
     }
-    b = __ballot_sync(kFull, leaf);
-    if (leaf) {
-        const int pos = npp + __popc(b & lt);
-        S.pp_begin[pos] = max(l0, 0);
-        S.pp_end[pos] = min(l1, n_bodies);
-        S.pp_mask[pos] = mk;
+    __device__ __forceinline__ void add_leaf(bool on, uint32_t b, uint32_t lt, int l0, int l1, uint32_t mk) {
+        if (on) {
+            const int pos = npp + __popc(b & lt);
+            S.pp_begin[pos] = min(max(l0, 0), n_bodies);
+            S.pp_end[pos] = max(S.pp_begin[pos], min(l1, n_bodies));
+            S.pp_mask[pos] = mk;
+        }
+        npp += __popc(b);
     }
-    npp += __popc(b);
+    // each round appends at most 32 leaves: evaluated before the next one could overflow the list
+    __device__ __forceinline__ void end_round() {
+        if (npp > kLeafFlush) flush_leaves();
+    }
+    __device__ __forceinline__ void finish() {
+        flush_full();
+        flush_part();
+        if (npp > 0) flush_leaves();
+        for (int k = 0; k < kLeafSets; ++k) {
+            const float *mine = sets + k * 96 + lane;
+            ax += mine[0];
+            ay += mine[32];
+            az += mine[64];
+        }
+    }
+};
+
+// Where they go in bh_team_kernel: the same lists, handed to the team's other warps at the same
+// points at which bh_kernel evaluates them.
+struct NodeList {
+    int count, all;  // all: accepted by every target; count < 0: the walk is done
+    int node[64];
+    uint32_t mask[64];
+};
+struct LeafList {
+    int count, pad;
+    int begin[kList], end[kList];
+    uint32_t mask[kList];
+};
+constexpr int kRing = 4;                     // node lists in flight; leaf lists: kLeafRing
+constexpr int kLeafRing = 8;
+constexpr int kTeamWarps = 2 + kLeafSets;    // walker, node evaluator, one warp per leaf set
+constexpr int kTeamThreads = 32 * kTeamWarps;
+constexpr int kTeamBlocks = 4;               // resident per SM, by shared memory
+
+template<int PAY, int PART>
+struct TeamSmem {
+    int2 stack[kTraverseStack];
+    float4 tpos[32];
+    float4 pay[(PART + 1) * PAY];            // (at least 32) the node evaluator's staged payloads, then the null payload
+    float4 tile[kLeafSets][32];              // the leaf warps' source bodies
+    NodeList nodes[kRing];
+    LeafList leaf[kLeafRing];
+    int full_node[kFullSlab];                // the walker's open lists
+    int part_node[PART];
+    uint32_t part_mask[PART];
+    int pp_begin[kList], pp_end[kList];
+    uint32_t pp_mask[kList];
+    int mixed_node[kList];
+    uint32_t mixed_mask[kList];
+    unsigned long long node_ready[kRing], node_free[kRing], leaf_ready[kLeafRing], leaf_free[kLeafRing];  // mbarriers
+    int abandon;                             // a wait ran out: every warp leaves
+};
+
+__device__ __forceinline__ void mbar_init(unsigned long long *bar, unsigned count) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"((uint32_t) __cvta_generic_to_shared(bar)), "r"(count) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(unsigned long long *bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"((uint32_t) __cvta_generic_to_shared(bar)) : "memory");
+}
+__device__ __forceinline__ bool mbar_try_wait(unsigned long long *bar, unsigned parity) {
+    unsigned ok;
+    asm volatile("{\n .reg .pred q;\n mbarrier.try_wait.parity.shared::cta.b64 q, [%1], %2;\n selp.u32 %0, 1, 0, q;\n}"
+                 : "=r"(ok) : "r"((uint32_t) __cvta_generic_to_shared(bar)), "r"(parity) : "memory");
+    return ok != 0;
+}
+// Waits until the barrier's phase `parity` is over, at most kTeamWaits tries and not once the team is abandoned. A
+// wait that runs out abandons the team with kErrTraverseLimit. Uniform over the warp.
+constexpr int kTeamWaits = 1 << 24;
+__device__ __forceinline__ bool team_wait(unsigned long long *bar, unsigned parity, int *abandon, uint32_t *err) {
+    for (int k = 0; k < kTeamWaits; ++k) {
+        if (__all_sync(kFull, mbar_try_wait(bar, parity))) return true;
+        if (__any_sync(kFull, *(volatile int *) abandon != 0)) return false;
+    }
+    if ((threadIdx.x & 31) == 0) {
+        atomicOr(err, (uint32_t) kErrTraverseLimit);
+        *(volatile int *) abandon = 1;
+    }
+    __syncwarp();
+    return false;
+}
+
+template<int ORDER, int PART>
+struct TeamSink {
+    static constexpr int PAY = NodeLayout<ORDER>::PAY;
+    TeamSmem<PAY, PART> &S;
+    uint32_t *err;
+    int lane, n_bodies;
+    int nfull = 0, npart = 0, npp = 0;
+    int node_lists = 0, leaf_lists = 0;  // lists handed over
+    bool lost = false;                   // the team was abandoned: nothing is handed over any more
+
+    __device__ __forceinline__ NodeList *open_nodes() {
+        const int slot = node_lists % kRing, turn = node_lists / kRing;
+        if (lost || (turn > 0 && !team_wait(&S.node_free[slot], (turn - 1) & 1, &S.abandon, err))) {
+            lost = true;
+            return nullptr;
+        }
+        return &S.nodes[slot];
+    }
+    __device__ __forceinline__ void hand_nodes() {
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&S.node_ready[node_lists % kRing]);
+        ++node_lists;
+    }
+    __device__ __forceinline__ void flush_full() {
+        if (nfull > 0)
+            if (NodeList *l = open_nodes()) {
+                if (lane == 0) {
+                    l->count = nfull;
+                    l->all = 1;
+                }
+                if (lane < nfull) l->node[lane] = S.full_node[lane];
+                hand_nodes();
+            }
+        nfull = 0;
+        __syncwarp();
+    }
+    __device__ __forceinline__ void flush_part() {
+        if (npart > 0)
+            if (NodeList *l = open_nodes()) {
+                if (lane == 0) {
+                    l->count = npart;
+                    l->all = 0;
+                }
+                for (int k = lane; k < npart; k += 32) {
+                    l->node[k] = S.part_node[k];
+                    l->mask[k] = S.part_mask[k];
+                }
+                hand_nodes();
+            }
+        npart = 0;
+        __syncwarp();
+    }
+    __device__ __forceinline__ void hand_leaves(int count) {
+        const int slot = leaf_lists % kLeafRing, turn = leaf_lists / kLeafRing;
+        if (lost || (turn > 0 && !team_wait(&S.leaf_free[slot], (turn - 1) & 1, &S.abandon, err))) {
+            lost = true;
+            return;
+        }
+        LeafList &l = S.leaf[slot];
+        if (lane == 0) l.count = count;
+        for (int k = lane; k < count; k += 32) {
+            l.begin[k] = S.pp_begin[k];
+            l.end[k] = S.pp_end[k];
+            l.mask[k] = S.pp_mask[k];
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&S.leaf_ready[slot]);
+        ++leaf_lists;
+    }
+    __device__ __forceinline__ void flush_leaves() {
+        flush_full();  // as the one-warp form does
+        if (npp > 0) hand_leaves(npp);
+        npp = 0;
+        __syncwarp();
+    }
+    __device__ __forceinline__ void add_full(bool on, uint32_t b, uint32_t lt, int c) {
+        if (nfull + __popc(b) > kFullSlab) flush_full();
+        if (on) S.full_node[nfull + __popc(b & lt)] = c;
+        nfull += __popc(b);
+    }
+    __device__ __forceinline__ void add_part(bool on, uint32_t b, uint32_t lt, int c, uint32_t mk) {
+        if (npart + __popc(b) > PART) flush_part();
+        if (on) {
+            const int slot = npart + __popc(b & lt);
+            S.part_node[slot] = c;
+            S.part_mask[slot] = mk;
+        }
+        npart += __popc(b);
+    }
+    __device__ __forceinline__ void add_leaf(bool on, uint32_t b, uint32_t lt, int l0, int l1, uint32_t mk) {
+        if (on) {
+            const int pos = npp + __popc(b & lt);
+            S.pp_begin[pos] = min(max(l0, 0), n_bodies);
+            S.pp_end[pos] = max(S.pp_begin[pos], min(l1, n_bodies));
+            S.pp_mask[pos] = mk;
+        }
+        npp += __popc(b);
+    }
+    __device__ __forceinline__ void end_round() {
+        if (npp > kLeafFlush) flush_leaves();
+    }
+    // the last lists, then one for each other warp that ends its work
+    __device__ __forceinline__ void finish() {
+        flush_full();
+        flush_part();
+        flush_leaves();
+        if (NodeList *l = open_nodes()) {
+            if (lane == 0) l->count = -1;
+            hand_nodes();
+        }
+        for (int set = 0; set < kLeafSets; ++set) hand_leaves(-1);
+    }
+};
+
+// Classified entries of one round, appended to the sink's lists (warp-uniform control flow):
+// acc / part are accepted nodes (target mask mk for part), leaf is an opened leaf (body range
+// l0..l1, mask mk), open an opened internal node (children c + 1 and l0, mask mk), mixed a node
+// still to be resolved per target.
+template<class Sink>
+__device__ __forceinline__ bool dispatch(Sink &sink, int2 *stack, int *mixed_node, uint32_t *mixed_mask, bool acc,
+                                         bool part, bool leaf, bool open, bool mixed, int c, uint32_t mk, int l0,
+                                         int l1, uint32_t lt, int lane, int &nmixed, int &top, uint32_t *err) {
+    uint32_t b = __ballot_sync(kFull, acc);
+    if (b) sink.add_full(acc, b, lt, c);
+    b = __ballot_sync(kFull, part);
+    if (b) sink.add_part(part, b, lt, c, mk);
+    b = __ballot_sync(kFull, leaf);
+    sink.add_leaf(leaf, b, lt, l0, l1, mk);
     b = __ballot_sync(kFull, mixed);
     if (mixed) {
         const int pos = nmixed + __popc(b & lt);
-        S.mixed_node[pos] = c;
-        S.mixed_mask[pos] = mk;
+        mixed_node[pos] = c;
+        mixed_mask[pos] = mk;
     }
     nmixed += __popc(b);
     b = __ballot_sync(kFull, open);
@@ -291,10 +672,143 @@ __device__ __forceinline__ bool dispatch(WarpSmem<NodeLayout<ORDER>::PAY, PART> 
         top += 2 * __popc(b);
     }
     __syncwarp();
-    // each round appends at most 32 leaves: evaluate before the next one could overflow the list
-    if (npp > kList - 32) flush_pp<EPS0, NodeLayout<ORDER>::PAY, PART>(S, npp, bodies, p, eps, lane, ax, ay, az, gpp);
+    sink.end_round();
     return abandoned;
 }
+
+// The walk of one group from `root` by one warp: `full` masks its valid targets, lo / hi is their
+// box, tpos their positions.
+template<class Sink>
+__device__ __forceinline__ void walk(Sink &sink, const NodeArrays &nodes, int num_nodes, int root, uint32_t full,
+                                     const float lo[3], const float hi[3], const float4 *tpos, int2 *stack,
+                                     int *mixed_node, uint32_t *mixed_mask, int64_t round_limit, uint32_t lt, int lane,
+                                     uint32_t *err) {
+    const float4 *__restrict__ mac = nodes.mac;
+    const int2 *__restrict__ link = nodes.link;
+    int top = 0, nmixed = 0;
+    if (num_nodes > 0 && root >= 0 && root < num_nodes) {
+        if (lane == 0) stack[0] = make_int2(root, (int) full);
+        top = 1;
+    } else if (num_nodes > 0 && lane == 0) {
+        atomicOr(err, (uint32_t) kErrTraverseLimit);  // a group without a valid tree root
+    }
+    __syncwarp();
+    int64_t rounds = 0;
+    while (top > 0 || nmixed > 0) {
+        if (++rounds > round_limit) {
+            if (lane == 0) atomicOr(err, (uint32_t) kErrTraverseLimit);
+            break;
+        }
+        if (top > 0) {
+            // ---- 1. pop up to 32 entries and classify them lane-parallel ----
+            const int k = min(32, top);
+            const int base = top - k;
+            top = base;
+            int c = 0, l0 = 0, l1 = -1, cls = kNone;
+            uint32_t m = 0;
+            if (lane < k) {
+                const int2 e = stack[base + lane];
+                c = e.x;
+                m = (uint32_t) e.y;
+                const float4 mc = __ldg(mac + c);
+                const int2 lk = __ldg(link + c);
+                l0 = lk.x;
+                l1 = lk.y;
+                // nearest box point and farthest box corner, per axis, with the reference's rounding
+                const float nx = fsub(fminf(fmaxf(mc.x, lo[0]), hi[0]), mc.x);
+                const float ny = fsub(fminf(fmaxf(mc.y, lo[1]), hi[1]), mc.y);
+                const float nz = fsub(fminf(fmaxf(mc.z, lo[2]), hi[2]), mc.z);
+                const float fx = fmaxf(fabsf(fsub(lo[0], mc.x)), fabsf(fsub(hi[0], mc.x)));
+                const float fy = fmaxf(fabsf(fsub(lo[1], mc.y)), fabsf(fsub(hi[1], mc.y)));
+                const float fz = fmaxf(fabsf(fsub(lo[2], mc.z)), fabsf(fsub(hi[2], mc.z)));
+                const float dmin2 = fadd(fadd(fmul(nx, nx), fmul(ny, ny)), fmul(nz, nz));
+                const float dmax2 = fadd(fadd(fmul(fx, fx), fmul(fy, fy)), fmul(fz, fz));
+                if (!(mc.w == mc.w)) cls = kOpenAll;  // NaN threshold: never approximated
+                else if (dmin2 >= mc.w) cls = kAcceptAll;
+                else if (dmax2 < mc.w) cls = kOpenAll;
+                else cls = kMixed;
+            }
+            __syncwarp();  // popped entries are read before children overwrite them
+            const bool is_leaf_open = cls == kOpenAll && l1 >= 0;
+            const bool is_int_open = cls == kOpenAll && l1 < 0 && l0 > c + 1 && l0 < num_nodes;
+            if (cls == kOpenAll && l1 < 0 && !is_int_open) atomicOr(err, (uint32_t) kErrTraverseLimit);
+            if (dispatch(sink, stack, mixed_node, mixed_mask, cls == kAcceptAll && m == full,
+                         cls == kAcceptAll && m != full, is_leaf_open, is_int_open, cls == kMixed, c, m, l0, l1, lt,
+                         lane, nmixed, top, err)) {
+                top = 0;
+                nmixed = 0;
+            }
+        }
+        if (nmixed >= 32 || (top == 0 && nmixed > 0)) {
+            // ---- 2. resolve up to 32 mixed nodes: per-target MAC, lane-parallel over nodes ----
+            const int k = min(32, nmixed);
+            const int base = nmixed - k;
+            nmixed = base;
+            int c = 0, l0 = 0, l1 = -1;
+            uint32_t A = 0, O = 0;
+            if (lane < k) {
+                c = mixed_node[base + lane];
+                const uint32_t m = mixed_mask[base + lane];
+                const float4 mc = __ldg(mac + c);
+                const int2 lk = __ldg(link + c);
+                l0 = lk.x;
+                l1 = lk.y;
+                uint32_t bits = 0;
+#pragma unroll 8
+                for (int t = 0; t < 32; ++t) {
+                    const float4 tp = tpos[t];
+                    bits |= (ref_dist2(tp.x, tp.y, tp.z, mc) >= mc.w) ? (1u << t) : 0u;
+                }
+                A = bits & m;
+                O = m & ~A;
+            }
+            __syncwarp();
+            const bool is_int_open = O != 0 && l1 < 0 && l0 > c + 1 && l0 < num_nodes;
+            if (O != 0 && l1 < 0 && !is_int_open) atomicOr(err, (uint32_t) kErrTraverseLimit);
+            const bool is_acc = A != 0 && A == full;
+            const bool is_part = A != 0 && A != full;
+            // an entry can be accepted by some targets and opened by others: append both parts
+            if (dispatch(sink, stack, mixed_node, mixed_mask, is_acc, is_part, false, false, false, c, A, l0, l1, lt,
+                         lane, nmixed, top, err) ||
+                dispatch(sink, stack, mixed_node, mixed_mask, false, false, O != 0 && l1 >= 0, is_int_open, false, c,
+                         O, l0, l1, lt, lane, nmixed, top, err)) {
+                top = 0;
+                nmixed = 0;
+            }
+        }
+    }
+}
+
+// Per axis, the box of the warp's valid targets (every lane gets it).
+__device__ __forceinline__ void target_box(float4 p, bool valid, float lo[3], float hi[3]) {
+    lo[0] = valid ? p.x : FLT_MAX; lo[1] = valid ? p.y : FLT_MAX; lo[2] = valid ? p.z : FLT_MAX;
+    hi[0] = valid ? p.x : -FLT_MAX; hi[1] = valid ? p.y : -FLT_MAX; hi[2] = valid ? p.z : -FLT_MAX;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            lo[k] = fminf(lo[k], __shfl_xor_sync(kFull, lo[k], o));
+            hi[k] = fmaxf(hi[k], __shfl_xor_sync(kFull, hi[k], o));
+        }
+    }
+}
+
+// Adds a group's (particle-particle, node-particle) interactions to the pass's and its instance's.
+__device__ __forceinline__ void add_counts(unsigned long long *counts, unsigned long long *inst_counts, int inst,
+                                           unsigned pp, unsigned np) {
+    if (counts) {
+        atomicAdd(counts + 0, (unsigned long long) pp);
+        atomicAdd(counts + 1, (unsigned long long) np);
+    }
+    if (inst_counts && inst >= 0) {
+        atomicAdd(inst_counts + 2 * (int64_t) inst, (unsigned long long) pp);
+        atomicAdd(inst_counts + 2 * (int64_t) inst + 1, (unsigned long long) np);
+    }
+}
+
+// A valid tree needs fewer chunk rounds than it has nodes for one group; the cap only bounds the
+// work on a corrupted tree.
+__device__ __forceinline__ int64_t walk_rounds(int num_nodes) { return 4 * (int64_t) num_nodes + 64; }
 
 template<int ORDER, bool EPS0, int THREADS, int PART>
 __global__ void __launch_bounds__(THREADS, kResidentThreads / THREADS) bh_kernel(NodeArrays nodes, const int *__restrict__ num_nodes_p,
@@ -308,20 +822,14 @@ __global__ void __launch_bounds__(THREADS, kResidentThreads / THREADS) bh_kernel
                                                          int num_group_tasks, const int *__restrict__ inst_root,
                                                          unsigned long long *__restrict__ inst_counts) {
     constexpr int PAY = NodeLayout<ORDER>::PAY;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
     WarpSmem<PAY, PART> &S = reinterpret_cast<WarpSmem<PAY, PART> *>(smem_raw)[warp];
-    int2 *stack = stack_base + ((int64_t) blockIdx.x * (THREADS / 32) + warp) * kTraverseStack;
-    const float4 *__restrict__ mac = nodes.mac;
-    const int2 *__restrict__ link = nodes.link;
-    const float4 *__restrict__ pay = nodes.pay;
+    int2 *stack = stack_base + ((int64_t) blockIdx.x * (THREADS / 32) + warp) * kWarpScratch;
     const int num_nodes = *num_nodes_p;
     const int num_groups = groups ? num_group_tasks : (n_targets + 31) / 32;
     const uint32_t lt = lanemask_lt();
-    // A valid tree needs fewer chunk rounds than it has nodes for one group; the cap only bounds
-    // the work on a corrupted tree.
-    const int64_t round_limit = 4 * (int64_t) num_nodes + 64;
-    unsigned cpp = 0, cnp = 0;
+    const int64_t round_limit = walk_rounds(num_nodes);
 
     while (true) {
         int g = 0;
@@ -340,145 +848,135 @@ __global__ void __launch_bounds__(THREADS, kResidentThreads / THREADS) bh_kernel
         const bool valid = lane < count && i < n_targets;
         const float4 p = valid ? targets[i] : make_float4(0.f, 0.f, 0.f, 0.f);
         const uint32_t full = __ballot_sync(kFull, valid);
-        float lo[3] = {valid ? p.x : FLT_MAX, valid ? p.y : FLT_MAX, valid ? p.z : FLT_MAX};
-        float hi[3] = {valid ? p.x : -FLT_MAX, valid ? p.y : -FLT_MAX, valid ? p.z : -FLT_MAX};
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                lo[k] = fminf(lo[k], __shfl_xor_sync(kFull, lo[k], o));
-                hi[k] = fmaxf(hi[k], __shfl_xor_sync(kFull, hi[k], o));
-            }
-        }
+        float lo[3], hi[3];
+        target_box(p, valid, lo, hi);
         S.tpos[lane] = p;
-        // the null payload: no mass and no moments at 1e30 on every axis, where the squared
-        // distance from any target with coordinates below 1e29 in magnitude overflows to
-        // infinity, so that every factor of the term is exactly zero and it adds nothing
-        if (lane < PAY) S.part_pay[PART * PAY + lane] = lane == 0 ? make_float4(1e30f, 1e30f, 1e30f, 0.f)
-                                                                  : make_float4(0.f, 0.f, 0.f, 0.f);
-        int top = 0, nfull = 0, npart = 0, npp = 0, nmixed = 0;
-        if (num_nodes > 0 && root >= 0 && root < num_nodes) {
-            if (lane == 0) stack[0] = make_int2(root, (int) full);
-            top = 1;
-        } else if (num_nodes > 0 && lane == 0) {
-            atomicOr(err, (uint32_t) kErrTraverseLimit);  // a group without a valid tree root
-        }
-        __syncwarp();
-        float ax = 0.f, ay = 0.f, az = 0.f;
-        unsigned gnp = 0, gpp = 0;  // this group's interaction counts (kept for valid targets only)
-        int64_t rounds = 0;
-
-        while (top > 0 || nmixed > 0) {
-            if (++rounds > round_limit) {
-                if (lane == 0) atomicOr(err, (uint32_t) kErrTraverseLimit);
-                break;
-            }
-            if (top > 0) {
-                // ---- 1. pop up to 32 entries and classify them lane-parallel ----
-                const int k = min(32, top);
-                const int base = top - k;
-                top = base;
-                int c = 0, l0 = 0, l1 = -1, cls = kNone;
-                uint32_t m = 0;
-                if (lane < k) {
-                    const int2 e = stack[base + lane];
-                    c = e.x;
-                    m = (uint32_t) e.y;
-                    const float4 mc = __ldg(mac + c);
-                    const int2 lk = __ldg(link + c);
-                    l0 = lk.x;
-                    l1 = lk.y;
-                    // nearest box point and farthest box corner, per axis, with the reference's rounding
-                    const float nx = fsub(fminf(fmaxf(mc.x, lo[0]), hi[0]), mc.x);
-                    const float ny = fsub(fminf(fmaxf(mc.y, lo[1]), hi[1]), mc.y);
-                    const float nz = fsub(fminf(fmaxf(mc.z, lo[2]), hi[2]), mc.z);
-                    const float fx = fmaxf(fabsf(fsub(lo[0], mc.x)), fabsf(fsub(hi[0], mc.x)));
-                    const float fy = fmaxf(fabsf(fsub(lo[1], mc.y)), fabsf(fsub(hi[1], mc.y)));
-                    const float fz = fmaxf(fabsf(fsub(lo[2], mc.z)), fabsf(fsub(hi[2], mc.z)));
-                    const float dmin2 = fadd(fadd(fmul(nx, nx), fmul(ny, ny)), fmul(nz, nz));
-                    const float dmax2 = fadd(fadd(fmul(fx, fx), fmul(fy, fy)), fmul(fz, fz));
-                    if (!(mc.w == mc.w)) cls = kOpenAll;  // NaN threshold: never approximated
-                    else if (dmin2 >= mc.w) cls = kAcceptAll;
-                    else if (dmax2 < mc.w) cls = kOpenAll;
-                    else cls = kMixed;
-                }
-                __syncwarp();  // popped entries are read before children overwrite them
-                const bool is_leaf_open = cls == kOpenAll && l1 >= 0;
-                const bool is_int_open = cls == kOpenAll && l1 < 0 && l0 > c + 1 && l0 < num_nodes;
-                if (cls == kOpenAll && l1 < 0 && !is_int_open) atomicOr(err, (uint32_t) kErrTraverseLimit);
-                if (dispatch<ORDER, EPS0, PART>(S, pay, bodies, stack, cls == kAcceptAll && m == full,
-                                          cls == kAcceptAll && m != full, is_leaf_open, is_int_open, cls == kMixed,
-                                          c, m, l0, l1, n_bodies, lt, lane, nfull, npart, npp, nmixed, top, p, eps,
-                                          ax, ay, az, gnp, gpp, err)) {
-                    top = 0;
-                    nmixed = 0;
-                }
-            }
-            if (nmixed >= 32 || (top == 0 && nmixed > 0)) {
-                // ---- 2. resolve up to 32 mixed nodes: per-target MAC, lane-parallel over nodes ----
-                const int k = min(32, nmixed);
-                const int base = nmixed - k;
-                nmixed = base;
-                int c = 0, l0 = 0, l1 = -1;
-                uint32_t A = 0, O = 0;
-                if (lane < k) {
-                    c = S.mixed_node[base + lane];
-                    const uint32_t m = S.mixed_mask[base + lane];
-                    const float4 mc = __ldg(mac + c);
-                    const int2 lk = __ldg(link + c);
-                    l0 = lk.x;
-                    l1 = lk.y;
-                    uint32_t bits = 0;
-#pragma unroll 8
-                    for (int t = 0; t < 32; ++t) {
-                        const float4 tp = S.tpos[t];
-                        bits |= (ref_dist2(tp.x, tp.y, tp.z, mc) >= mc.w) ? (1u << t) : 0u;
-                    }
-                    A = bits & m;
-                    O = m & ~A;
-                }
-                __syncwarp();
-                const bool is_int_open = O != 0 && l1 < 0 && l0 > c + 1 && l0 < num_nodes;
-                if (O != 0 && l1 < 0 && !is_int_open) atomicOr(err, (uint32_t) kErrTraverseLimit);
-                const bool is_acc = A != 0 && A == full;
-                const bool is_part = A != 0 && A != full;
-                // an entry can be accepted by some targets and opened by others: append both parts
-                if (dispatch<ORDER, EPS0, PART>(S, pay, bodies, stack, is_acc, is_part, false, false, false, c, A, l0,
-                                          l1, n_bodies, lt, lane, nfull, npart, npp, nmixed, top, p, eps, ax, ay,
-                                          az, gnp, gpp, err) ||
-                    dispatch<ORDER, EPS0, PART>(S, pay, bodies, stack, false, false, O != 0 && l1 >= 0, is_int_open, false,
-                                          c, O, l0, l1, n_bodies, lt, lane, nfull, npart, npp, nmixed, top, p, eps,
-                                          ax, ay, az, gnp, gpp, err)) {
-                    top = 0;
-                    nmixed = 0;
-                }
-            }
-        }
-        flush_full<ORDER, EPS0, PART>(S, nfull, p, eps, ax, ay, az, gnp);
-        flush_part<ORDER, EPS0, PART>(S, npart, p, eps, lane, ax, ay, az, gnp);
-        flush_pp<EPS0, PAY, PART>(S, npp, bodies, p, eps, lane, ax, ay, az, gpp);
-        if (valid) acc[i] = make_float4(G * ax, G * ay, G * az, 0.f);
-        if (valid) {
-            cnp += gnp;
-            cpp += gpp;
-        }
-        if (inst_counts && inst >= 0) {
-            const unsigned ipp = __reduce_add_sync(kFull, valid ? gpp : 0u);
-            const unsigned inp = __reduce_add_sync(kFull, valid ? gnp : 0u);
-            if (lane == 0) {
-                atomicAdd(inst_counts + 2 * (int64_t) inst, (unsigned long long) ipp);
-                atomicAdd(inst_counts + 2 * (int64_t) inst + 1, (unsigned long long) inp);
-            }
-        }
+        write_null_payload<PAY>(S.part_pay + PART * PAY, lane);
+        WarpSink<ORDER, EPS0, PART> sink{S, nodes.pay, bodies, p, eps, lane, n_bodies};
+        sink.sets = reinterpret_cast<float *>(stack + kTraverseStack);
+        sink.clear();
+        walk(sink, nodes, num_nodes, root, full, lo, hi, S.tpos, stack, S.mixed_node, S.mixed_mask, round_limit, lt,
+             lane, err);
+        sink.finish();
+        if (valid) acc[i] = make_float4(G * sink.ax, G * sink.ay, G * sink.az, 0.f);
+        // interaction counts of the valid targets
+        const unsigned spp = __reduce_add_sync(kFull, valid ? S.pair_count[lane] : 0u);
+        const unsigned snp = __reduce_add_sync(kFull, valid ? S.node_count[lane] : 0u);
+        if (lane == 0) add_counts(counts, inst_counts, inst, spp, snp);
         __syncwarp();
     }
-    if (counts) {
-        const unsigned spp = __reduce_add_sync(kFull, cpp);
-        const unsigned snp = __reduce_add_sync(kFull, cnp);
-        if (lane == 0) {
-            atomicAdd(counts + 0, (unsigned long long) spp);
-            atomicAdd(counts + 1, (unsigned long long) snp);
+}
+
+// One block per group, for launches whose groups alone do not fill the GPU (team_groups): warp 0 walks, warp 1
+// evaluates the approximated nodes, warp 2 + k the leaf lists of set k. Bound by the walk's chain of
+// rounds (two dependent loads and several hundred instructions each); with one warp per group the
+// leaf pairs came on top of it at 6 to 11 cycles per instruction, one warp per scheduler. Traversal
+// time, one warp / team: 1,023-body Plummer 92 / 40 us, 10,000-body ball 427 / 115 us, 10,000-body
+// Plummer 607 / 135 us, 100,003 bodies at leaf 64 and theta 0.3 6.7 / 3.9 ms.
+template<int ORDER, bool EPS0, int PART>
+__global__ void __launch_bounds__(kTeamThreads, kTeamBlocks)
+    bh_team_kernel(NodeArrays nodes, const int *__restrict__ num_nodes_p, const float4 *__restrict__ bodies, int n_bodies,
+                   const float4 *__restrict__ targets, int n_targets, float G, float eps, float4 *__restrict__ acc,
+                   unsigned long long *__restrict__ counts, uint32_t *__restrict__ err, const int4 *__restrict__ groups,
+                   const int *__restrict__ inst_root, unsigned long long *__restrict__ inst_counts) {
+    constexpr int PAY = NodeLayout<ORDER>::PAY;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    TeamSmem<PAY, PART> &S = *reinterpret_cast<TeamSmem<PAY, PART> *>(smem_raw);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int g = blockIdx.x;
+    int first = g * 32, count = min(32, n_targets - g * 32), root = 0, inst = -1;
+    if (groups) {
+        const int4 ge = groups[g];
+        first = ge.x;
+        count = ge.y;
+        inst = ge.z;
+        root = inst_root[inst];
+    }
+    const int i = first + lane;
+    const bool valid = lane < count && i < n_targets;
+    const float4 p = valid ? targets[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+    if (threadIdx.x == 0) {
+        for (int k = 0; k < kRing; ++k) {
+            mbar_init(&S.node_ready[k], 1);
+            mbar_init(&S.node_free[k], 1);
         }
+        for (int k = 0; k < kLeafRing; ++k) {
+            mbar_init(&S.leaf_ready[k], 1);
+            mbar_init(&S.leaf_free[k], 1);
+        }
+        S.abandon = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 0) S.tpos[lane] = p;
+    if (warp == 1) write_null_payload<PAY>(S.pay + PART * PAY, lane);
+    __syncthreads();
+
+    float ax = 0.f, ay = 0.f, az = 0.f;
+    unsigned taken = 0;
+    if (warp == 0) {
+        const int num_nodes = *num_nodes_p;
+        const uint32_t full = __ballot_sync(kFull, valid);
+        float lo[3], hi[3];
+        target_box(p, valid, lo, hi);
+        TeamSink<ORDER, PART> sink{S, err, lane, n_bodies};
+        walk(sink, nodes, num_nodes, root, full, lo, hi, S.tpos, S.stack, S.mixed_node, S.mixed_mask,
+             walk_rounds(num_nodes), lanemask_lt(), lane, err);
+        sink.finish();
+    } else if (warp == 1) {
+        for (int q = 0;; ++q) {
+            const int slot = q % kRing;
+            if (!team_wait(&S.node_ready[slot], (q / kRing) & 1, &S.abandon, err)) break;
+            const NodeList &l = S.nodes[slot];
+            const int n = l.count;
+            if (n < 0) break;
+            for (int k = lane; k < n; k += 32) stage_node<PAY>(S.pay + k * PAY, nodes.pay, l.node[k]);
+            cp_async_wait_all();
+            __syncwarp();
+            if (l.all) {
+                full_terms<ORDER, EPS0>(S.pay, n, p, eps, lane, ax, ay, az);
+                taken += (unsigned) n;
+            } else {
+                taken += part_terms<ORDER, EPS0, PART>(S.pay, l.mask, n, p, eps, lane, ax, ay, az);
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&S.node_free[slot]);
+        }
+    } else {
+        for (int q = warp - 2;; q += kLeafSets) {
+            const int slot = q % kLeafRing;
+            if (!team_wait(&S.leaf_ready[slot], (q / kLeafRing) & 1, &S.abandon, err)) break;
+            const LeafList &l = S.leaf[slot];
+            const int n = l.count;
+            if (n < 0) break;
+            taken += leaf_terms<EPS0>(l.begin, l.end, l.mask, n, bodies, S.tile[warp - 2], p, eps, lane, ax, ay, az);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&S.leaf_free[slot]);
+        }
+    }
+    // the sets meet in the buffers that each warp staged its sources in (32 float4 or more each)
+    __syncwarp();
+    if (warp > 0) {
+        float4 *mine = warp == 1 ? S.pay : S.tile[warp - 2];
+        mine[lane] = make_float4(ax, ay, az, __uint_as_float(taken));
+    }
+    __syncthreads();
+    if (warp == 0) {
+        const float4 nodes_sum = S.pay[lane];
+        ax = nodes_sum.x;
+        ay = nodes_sum.y;
+        az = nodes_sum.z;
+        unsigned pairs = 0;
+        for (int k = 0; k < kLeafSets; ++k) {
+            const float4 v = S.tile[k][lane];
+            ax += v.x;
+            ay += v.y;
+            az += v.z;
+            pairs += __float_as_uint(v.w);
+        }
+        if (valid) acc[i] = make_float4(G * ax, G * ay, G * az, 0.f);
+        const unsigned spp = __reduce_add_sync(kFull, valid ? pairs : 0u);
+        const unsigned snp = __reduce_add_sync(kFull, valid ? __float_as_uint(nodes_sum.w) : 0u);
+        if (lane == 0) add_counts(counts, inst_counts, inst, spp, snp);
     }
 }
 
@@ -505,13 +1003,25 @@ int resident_warps(int device) {
     return sm_count(device) * blocks_per_sm<ORDER, EPS0, THREADS, PART>(device) * (THREADS / 32);
 }
 
+// Launches of at most this many groups run one team of warps per group, larger ones one warp per
+// group. The team form has one walking warp in eight, so it loses where the groups alone fill the
+// GPU; larger leaves shift work from the walk to the leaf warps and the line with it. Measured
+// (warp form over team form, traversal time, orders 1 and 2, theta 0.3 to 0.65, Plummer and ball):
+// leaf 8: 2.0-3.4 at 16k bodies, 1.1-1.6 at 49k, 0.9-1.15 at 65k; leaf 16: 1.06-1.8 at 65k,
+// 0.86-1.4 at 98k; leaf 32: 1.03-1.7 at 131k, 0.84-1.3 at 196k; leaf 64: 1.1-1.5 at 196k,
+// 0.98-1.2 at 262k. Leaves above 64 bodies give too few lists to share out: always one warp.
+int64_t team_groups(int device, int leaf) {
+    if (leaf > 64) return 0;
+    return (int64_t) sm_count(device) * (24 + 3 * leaf) / 4;
+}
+
 struct LaunchArgs {
     const NodeArrays *nodes;
     const int *num_nodes;
     const float4 *bodies;
     int n_bodies;
     const float4 *targets;
-    int nt;
+    int nt, leaf;
     float G, eps;
     float4 *acc;
     unsigned long long *counts;
@@ -524,15 +1034,35 @@ struct LaunchArgs {
     unsigned long long *inst_counts;
 };
 
+// The team kernel's dynamic shared memory is enabled on first use per device.
+template<int ORDER, bool EPS0, int PART>
+void launch_team(const LaunchArgs &a, int device) {
+    static bool ready[64] = {false};
+    constexpr size_t smem = sizeof(TeamSmem<NodeLayout<ORDER>::PAY, PART>);
+    auto kernel = bh_team_kernel<ORDER, EPS0, PART>;
+    if (device < 0 || device >= 64) device = 0;
+    if (!ready[device]) {
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
+        cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+        ready[device] = true;
+    }
+    kernel<<<(unsigned) a.ngroups, kTeamThreads, smem, a.s>>>(*a.nodes, a.num_nodes, a.bodies, a.n_bodies, a.targets,
+                                                              a.nt, a.G, a.eps, a.acc, a.counts, a.err, a.gtab,
+                                                              a.inst_root, a.inst_counts);
+}
+
 template<int ORDER, bool EPS0, int THREADS, int PART>
 void launch_variant(const LaunchArgs &a) {
     constexpr int kWarps = THREADS / 32;
     int device = 0;
     cudaGetDevice(&device);
+    if (a.ngroups <= team_groups(device, a.leaf)) {
+        launch_team<ORDER, EPS0, PART>(a, device);
+        return;
+    }
     int64_t blocks = (int64_t) sm_count(device) * blocks_per_sm<ORDER, EPS0, THREADS, PART>(device);
     blocks = std::min<int64_t>(blocks, a.ws->warps / kWarps);
-    const int64_t groups = a.gtab ? a.ngroups : (a.nt + 31) / 32;
-    blocks = std::min<int64_t>(blocks, (groups + kWarps - 1) / kWarps);
+    blocks = std::min<int64_t>(blocks, (a.ngroups + kWarps - 1) / kWarps);
     if (blocks < 1) blocks = 1;
     cudaMemsetAsync(a.ws->group_counter, 0, sizeof(unsigned), a.s);
     bh_kernel<ORDER, EPS0, THREADS, PART><<<(unsigned) blocks, THREADS, block_smem_bytes<ORDER, THREADS, PART>(), a.s>>>(
@@ -584,11 +1114,12 @@ int64_t traverse_resident_warps(int device) {
 bool traversal_shape_valid(int threads, int slab) { return (threads == 128 || threads == 256) && (slab == 32 || slab == 64); }
 
 void launch_bh_traverse(int order, const NodeArrays &nodes, const int *num_nodes, const float4 *bodies, int64_t n_bodies,
-                        const float4 *targets, int64_t n_targets, float G, float eps, float4 *acc,
+                        const float4 *targets, int64_t n_targets, int leaf, float G, float eps, float4 *acc,
                         unsigned long long *counts, TraverseWorkspace &ws, uint32_t *err, cudaStream_t s,
                         const int4 *gtab, int64_t ngroups, const int *inst_root, unsigned long long *inst_counts) {
     if (n_targets <= 0) return;
-    const LaunchArgs a{&nodes, num_nodes, bodies, (int) n_bodies, targets, (int) n_targets, G, eps, acc, counts, &ws,
+    if (!gtab) ngroups = (n_targets + 31) / 32;
+    const LaunchArgs a{&nodes, num_nodes, bodies, (int) n_bodies, targets, (int) n_targets, leaf, G, eps, acc, counts, &ws,
                        err, s, gtab, ngroups, inst_root, inst_counts};
     const bool ok = traversal_shape_valid(ws.threads, ws.slab);
     const int threads = ok ? ws.threads : 256, part = ok ? ws.slab : 64;
