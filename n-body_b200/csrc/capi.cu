@@ -503,7 +503,7 @@ int force_pass(nb_ctx *ctx, Marks &mk) {
     shard_slice(n, ctx->shard_rank, ctx->shard_world, &chunk, &first, &count);
     if (ctx->cfg.solver == NB_SOLVER_NAIVE) {
         mk.mark(kMorton); mk.mark(kSort); mk.mark(kGather); mk.mark(kBuild); mk.mark(kTraverse);
-        launch_direct_f32(ctx->pos, n, ctx->pos + first, count, ctx->cfg.G, ctx->cfg.epsilon, ctx->acc + first, s);
+        launch_direct_f32(ctx->pos, n, ctx->pos + first, count, n, ctx->cfg.G, ctx->cfg.epsilon, ctx->acc + first, s);
         ctx->have_tree = false;
         ctx->acc_is_bh = false;
         if (ctx->timing) ctx->times.launches += 1;
@@ -1052,7 +1052,7 @@ int nb_direct_device(nb_ctx *ctx, int64_t n, const void *d_bodies, int64_t nt, c
     if (n < 0 || nt < 0 || (n > 0 && !d_bodies) || (nt > 0 && (!d_targets || !d_acc)))
         return fail(ctx, NB_ERR_INVALID_ARGUMENT, "bad direct-sum arguments");
     if (precision == 32)
-        launch_direct_f32((const float4 *) d_bodies, n, (const float4 *) d_targets, nt, ctx->cfg.G, ctx->cfg.epsilon,
+        launch_direct_f32((const float4 *) d_bodies, n, (const float4 *) d_targets, nt, nt, ctx->cfg.G, ctx->cfg.epsilon,
                           (float4 *) d_acc, ctx->stream);
     else if (precision == 64)
         launch_direct_f64((const float4 *) d_bodies, n, (const float4 *) d_targets, nt, (double) ctx->cfg.G,

@@ -325,8 +325,10 @@ void launch_bh_traverse(int order, const NodeArrays &nodes, const int *num_nodes
 int64_t energy_parts(int64_t n);
 void launch_energy_f64(const float4 *bodies, const float4 *vel, int64_t n, double G, double eps, double *parts,
                        double *out, cudaStream_t s);
-void launch_direct_f32(const float4 *bodies, int64_t n, const float4 *targets, int64_t nt, float G, float eps,
-                       float4 *acc, cudaStream_t s);
+// shape_targets: the target count that the split of the work (and the order of the sums) is chosen
+// for; a shard of a body set passes the whole set's, so that it sums as an unsharded pass does.
+void launch_direct_f32(const float4 *bodies, int64_t n, const float4 *targets, int64_t nt, int64_t shape_targets,
+                       float G, float eps, float4 *acc, cudaStream_t s);
 void launch_direct_f64(const float4 *bodies, int64_t n, const float4 *targets, int64_t nt, double G, double eps,
                        double *acc3, cudaStream_t s);
 

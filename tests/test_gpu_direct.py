@@ -1,0 +1,84 @@
+"""Direct sums and energies at the remainders of their tiles, warps and clusters, against FP64 on the host.
+
+Tolerances: an FP32 term carries a reciprocal root good to about 2^-22 (cubed) and some ten roundings, an
+FP64 term some ten roundings of 2^-53, and sums of a few thousand terms add far less than that again;
+bounds are relative to the sum of the terms' magnitudes.
+"""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def reference(bodies, targets, eps):
+    d = bodies[None, :, :3].astype(np.float64) - targets[:, None, :3].astype(np.float64)
+    d2 = (d * d).sum(-1)
+    w = np.zeros_like(d2)
+    np.divide(bodies[None, :, 3].astype(np.float64), (d2 + eps) ** 1.5, out=w, where=d2 > 0)
+    terms = d * w[..., None]
+    return terms.sum(1), np.abs(terms).sum(1)
+
+
+@pytest.mark.parametrize("n,nt", [(1, 1), (2, 33), (255, 31), (256, 32), (257, 300), (1025, 1), (4097, 513), (20011, 64)])
+@pytest.mark.parametrize("eps", [0.0, 1e-4])
+def test_direct_sums(nb, n, nt, eps):
+    import torch
+
+    pm, _ = nb.scenarios.plummer(max(n, 8), seed=n + nt)
+    pm = pm[:n]
+    rng = np.random.default_rng(n)
+    targets = np.concatenate([pm, rng.uniform(-2, 2, (nt, 4)).astype(np.float32)])[-nt:] if n % 2 else pm[np.arange(nt) % n]
+    eps = float(np.float32(eps))
+    ref, size = reference(pm, targets, eps)
+    b, t = torch.from_numpy(pm).cuda(), torch.from_numpy(np.ascontiguousarray(targets)).cuda()
+    a32 = torch.zeros(nt, 4, device="cuda")
+    a64 = torch.zeros(nt, 3, device="cuda", dtype=torch.float64)
+    torch.cuda.synchronize()
+    with nb.NaiveSolver(None, nb.Gravity(1.0, eps)) as s:
+        s.direct_device(n, b.data_ptr(), nt, t.data_ptr(), a32.data_ptr(), 32)
+        s.direct_device(n, b.data_ptr(), nt, t.data_ptr(), a64.data_ptr(), 64)
+        s.synchronize()
+    assert (np.abs(a32.cpu().numpy()[:, :3] - ref) <= 4e-6 * size).all()
+    assert (np.abs(a64.cpu().numpy() - ref) <= 2e-14 * size).all()
+
+
+def test_wide_direct_sums(nb):
+    import torch
+
+    pm, _ = nb.scenarios.plummer(300, seed=3)
+    nt = 300_037  # one thread per target
+    t = torch.from_numpy(pm[np.arange(nt) % 300]).cuda()
+    b = torch.from_numpy(pm).cuda()
+    a32 = torch.zeros(nt, 4, device="cuda")
+    a64 = torch.zeros(nt, 3, device="cuda", dtype=torch.float64)
+    torch.cuda.synchronize()
+    ref, size = reference(pm, pm, float(np.float32(1e-4)))
+    with nb.NaiveSolver(None, nb.Gravity(1.0, 1e-4)) as s:
+        s.direct_device(300, b.data_ptr(), nt, t.data_ptr(), a32.data_ptr(), 32)
+        s.direct_device(300, b.data_ptr(), nt, t.data_ptr(), a64.data_ptr(), 64)
+        s.synchronize()
+    at = np.arange(nt) % 300
+    assert (np.abs(a32.cpu().numpy()[:, :3] - ref[at]) <= 4e-6 * size[at]).all()
+    assert (np.abs(a64.cpu().numpy() - ref[at]) <= 2e-14 * size[at]).all()
+
+
+@pytest.mark.parametrize("n", [1, 2, 255, 256, 257, 512, 513, 1024, 1025, 5000])
+@pytest.mark.parametrize("eps", [0.0, 1e-4])
+def test_energy(nb, n, eps):
+    pm, vel = nb.scenarios.plummer(max(n, 8), seed=n)
+    pm, vel = pm[:n].copy(), vel[:n]
+    if n > 300:
+        pm[300, :3] = pm[10, :3]  # coincident bodies in different tiles
+        pm[301, :3] = pm[300, :3]
+    eps = float(np.float32(eps))
+    p = pm.astype(np.float64)
+    u = 0.0
+    for i in range(n):
+        d2 = ((p[:, :3] - p[i, :3]) ** 2).sum(1)
+        on = d2 > 0
+        u += p[i, 3] * (p[on, 3] / np.sqrt(d2[on] + eps)).sum()
+    k = 0.5 * (p[:, 3] * (vel[:, :3].astype(np.float64) ** 2).sum(1)).sum()
+    with nb.NaiveSolver(pm, nb.Gravity(1.0, eps), vel) as s:
+        kinetic, potential = s.energy()
+    assert abs(kinetic - k) <= 1e-14 * k
+    assert abs(potential + 0.5 * u) <= 1e-14 * max(u, 1e-300)
