@@ -73,7 +73,8 @@ __global__ void __launch_bounds__(kThreads) seg_morton_kernel(const float4 *__re
                                                               uint64_t *__restrict__ codes,
                                                               uint32_t *__restrict__ hist) {
     __shared__ uint32_t sh[8 * 256];
-    for (int i = threadIdx.x; i < 8 * 256; i += blockDim.x) sh[i] = 0;
+    if (hist)
+        for (int i = threadIdx.x; i < 8 * 256; i += blockDim.x) sh[i] = 0;
     __syncthreads();
     const int64_t stride = (int64_t) gridDim.x * blockDim.x;
     for (int64_t i = (int64_t) blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
@@ -85,9 +86,11 @@ __global__ void __launch_bounds__(kThreads) seg_morton_kernel(const float4 *__re
         const float scale = gmax(gmax(dx, dy), dz);
         const uint64_t code = morton_code(__ldg(pos + i), mn, scale);
         codes[i] = code;
+        if (!hist) continue;
 #pragma unroll
         for (int d = 0; d < 8; ++d) atomicAdd(&sh[d * 256 + (uint32_t) ((code >> (8 * d)) & 255u)], 1u);
     }
+    if (!hist) return;
     __syncthreads();
     for (int i = threadIdx.x; i < 8 * 256; i += blockDim.x) {
         const uint32_t c = sh[i];
@@ -155,7 +158,6 @@ void launch_seg_bbox(const float4 *pos, const int2 *inst_range, int num_inst, in
 void launch_seg_morton(const float4 *pos, int64_t n, const int *inst_of, const uint32_t *inst_box, uint64_t *codes,
                        uint32_t *hist, cudaStream_t s) {
     if (n <= 0) return;
-    cudaMemsetAsync(hist, 0, 8 * 256 * sizeof(uint32_t), s);
     int64_t blocks = (n + kThreads * 4 - 1) / (kThreads * 4);
     blocks = blocks < 1 ? 1 : (blocks > 148 * 8 ? 148 * 8 : blocks);
     seg_morton_kernel<<<(unsigned) blocks, kThreads, 0, s>>>(pos, n, inst_of, inst_box, codes, hist);

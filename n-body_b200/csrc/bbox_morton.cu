@@ -62,7 +62,8 @@ __global__ void __launch_bounds__(kThreads) morton_hist_kernel(const float4 *__r
                                                                uint64_t *__restrict__ codes,
                                                                uint32_t *__restrict__ hist) {
     __shared__ uint32_t sh[8 * 256];
-    for (int i = threadIdx.x; i < 8 * 256; i += blockDim.x) sh[i] = 0;
+    if (hist)
+        for (int i = threadIdx.x; i < 8 * 256; i += blockDim.x) sh[i] = 0;
     float mn[3], mx[3];
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
@@ -76,9 +77,11 @@ __global__ void __launch_bounds__(kThreads) morton_hist_kernel(const float4 *__r
     for (int64_t i = (int64_t) blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
         const uint64_t code = morton_code(__ldg(pos + i), mn, scale);
         codes[i] = code;
+        if (!hist) continue;
 #pragma unroll
         for (int d = 0; d < 8; ++d) atomicAdd(&sh[d * 256 + (uint32_t) ((code >> (8 * d)) & 255u)], 1u);
     }
+    if (!hist) return;
     __syncthreads();
     for (int i = threadIdx.x; i < 8 * 256; i += blockDim.x) {
         uint32_t c = sh[i];
@@ -105,8 +108,7 @@ void launch_bbox_reduce(const float4 *pos, int64_t n, BBoxAccum *acc, cudaStream
 void launch_morton_hist(const float4 *pos, int64_t n, const BBoxAccum *acc, uint64_t *codes, uint32_t *hist,
                         cudaStream_t s) {
     if (n <= 0) return;
-    cudaMemsetAsync(hist, 0, 8 * 256 * sizeof(uint32_t), s);
-    morton_hist_kernel<<<grid_for(n, 4), kThreads, 0, s>>>(pos, n, acc, codes, hist);
+    morton_hist_kernel<<<grid_for(n, hist ? 4 : 1), kThreads, 0, s>>>(pos, n, acc, codes, hist);
 }
 
 }  // namespace nbg

@@ -83,7 +83,7 @@ struct nb_ctx {
     unsigned long long *inst_counts = nullptr;  // (particle-particle, node-particle) per instance
     uint64_t *ikeys = nullptr, *ikeys2 = nullptr;
     uint32_t *ivals = nullptr, *ivals2 = nullptr;
-    uint32_t *inst_offsets = nullptr, *inst_lookback = nullptr, *inst_tiles = nullptr;
+    uint32_t *inst_hist = nullptr, *inst_lookback = nullptr, *inst_tiles = nullptr;
     int inst_passes = 0;
     int64_t batch_body_cap = 0, batch_inst_cap = 0, batch_group_cap = 0;  // grow-only batch buffers
     int *group_first = nullptr;
@@ -180,7 +180,7 @@ int validate(nb_ctx *ctx, const nb_config *cfg) {
 void free_batch(nb_ctx *ctx) {
     dev_free(ctx->inst_of); dev_free(ctx->inst_root); dev_free(ctx->inst_theta2); dev_free(ctx->inst_box);
     dev_free(ctx->inst_range); dev_free(ctx->groups); dev_free(ctx->ikeys); dev_free(ctx->ikeys2);
-    dev_free(ctx->ivals); dev_free(ctx->ivals2); dev_free(ctx->inst_offsets); dev_free(ctx->inst_lookback);
+    dev_free(ctx->ivals); dev_free(ctx->ivals2); dev_free(ctx->inst_hist); dev_free(ctx->inst_lookback);
     dev_free(ctx->inst_tiles); dev_free(ctx->group_first); dev_free(ctx->inst_counts);
     ctx->batch_body_cap = ctx->batch_inst_cap = ctx->batch_group_cap = 0;
     ctx->num_inst = 0;
@@ -266,7 +266,8 @@ void free_buffers(nb_ctx *ctx) {
     free_dual(ctx);
     dev_free(ctx->pos); dev_free(ctx->vel); dev_free(ctx->acc); dev_free(ctx->pos2); dev_free(ctx->vel2);
     dev_free(ctx->id); dev_free(ctx->id2); dev_free(ctx->keys); dev_free(ctx->vals);
-    dev_free(ctx->sw.keys_alt); dev_free(ctx->sw.vals_alt); dev_free(ctx->sw.lookback);
+    dev_free(ctx->sw.keys_alt); dev_free(ctx->sw.vals_alt); dev_free(ctx->sw.hist);
+    ctx->sw.tile_counter = ctx->sw.lookback = nullptr;
     dev_free(ctx->tw.topo); dev_free(ctx->tw.parent); dev_free(ctx->tw.flags); dev_free(ctx->tw.visit);
     dev_free(ctx->tw.slot); dev_free(ctx->tw.chain);
     dev_free(ctx->tw.start); dev_free(ctx->tw.pre_base); dev_free(ctx->tw.scan_part);
@@ -292,7 +293,9 @@ int ensure_capacity(nb_ctx *ctx, int64_t n) {
     NB_TRY(dev_alloc(&ctx->vals, c), "alloc sort values");
     NB_TRY(dev_alloc(&ctx->sw.keys_alt, c), "alloc codes");
     NB_TRY(dev_alloc(&ctx->sw.vals_alt, c), "alloc sort values");
-    NB_TRY(dev_alloc(&ctx->sw.lookback, sort_lookback_words(c)), "alloc sort look-back");
+    uint32_t *sort_block = nullptr;
+    NB_TRY(dev_alloc(&sort_block, sort_words(c)), "alloc sort look-back");
+    place_sort(ctx->sw, sort_block);
     ctx->sw.capacity = c;
     NB_TRY(dev_alloc(&ctx->tw.topo, c), "alloc tree");
     NB_TRY(dev_alloc(&ctx->tw.parent, c), "alloc tree");
@@ -378,10 +381,10 @@ void collect_times(nb_ctx *ctx) {
 int64_t launches_per_pass(const nb_ctx *ctx, bool with_bbox, bool with_drift) {
     if (ctx->cfg.solver == NB_SOLVER_NAIVE) return 1 + (with_drift ? 1 : 0);
     // the dual path adds loadBalancedBreak to the same pipeline
-    // morton(1) + scan(1) + 8 sort passes + gather(1) + karras(1) + summarize(1) + emit(1)
+    // morton(1) + sort (8 passes, or 1 kernel) + gather(1) + karras(1) + scans(3) + summarize(1)
     // + root-leaf(1) + traverse(1)
-    int64_t k = 1 + 1 + 8 + 1 + 1 + 1 + 1 + 1 + 1;
-    if (ctx->n <= 1) k -= 3;  // no Karras internal nodes
+    int64_t k = 1 + (ctx->n > kSmallSort ? 8 : 1) + 1 + 1 + 3 + 1 + 1 + 1;
+    if (ctx->n <= 1) k -= 5;  // no Karras internal nodes
     if (ctx->cfg.solver == NB_SOLVER_DUAL_LINEAR_BVH) k += 2;  // loadBalancedBreak and the near-field kernel
     return k + (with_bbox ? 1 : 0) + (with_drift ? 1 : 0);
 }
@@ -449,18 +452,19 @@ int force_pass_batch(nb_ctx *ctx, Marks &mk) {
     cudaStream_t s = ctx->stream;
     launch_seg_bbox(ctx->pos, ctx->inst_range, ctx->num_inst, ctx->inst_bbox_slices, ctx->inst_box, s);
     mk.mark(kMorton);
-    launch_seg_morton(ctx->pos, n, ctx->inst_of, ctx->inst_box, ctx->keys, ctx->sw.hist, s);
+    NB_TRY(clear_sort(n, ctx->sw, s), "radix sort");
+    launch_seg_morton(ctx->pos, n, ctx->inst_of, ctx->inst_box, ctx->keys, n > kSmallSort ? ctx->sw.hist : nullptr, s);
     mk.mark(kSort);
-    NB_TRY(launch_radix_sort(ctx->keys, ctx->vals, n, ctx->sw, ctx->err, s), "radix sort");
+    NB_TRY(launch_radix_sort(ctx->keys, ctx->keys, ctx->vals, n, ctx->sw, ctx->err, s), "radix sort");
     launch_inst_keys(ctx->vals, n, ctx->inst_of, ctx->ikeys, s);
     const int64_t tiles = sort_tiles(n);
     cudaMemsetAsync(ctx->inst_lookback, 0, (size_t) ctx->inst_passes * tiles * 256 * sizeof(uint32_t), s);
     cudaMemsetAsync(ctx->inst_tiles, 0, 8 * sizeof(uint32_t), s);
-    launch_radix_pass(ctx->ikeys, nullptr, ctx->ikeys2, ctx->ivals, n, 0, ctx->inst_offsets, ctx->inst_lookback,
+    launch_radix_pass(ctx->ikeys, nullptr, ctx->ikeys2, ctx->ivals, n, 0, ctx->inst_hist, ctx->inst_lookback,
                       ctx->inst_tiles, ctx->err, s);
     const uint32_t *order = ctx->ivals;
     if (ctx->inst_passes == 2) {
-        launch_radix_pass(ctx->ikeys2, ctx->ivals, ctx->ikeys, ctx->ivals2, n, 1, ctx->inst_offsets,
+        launch_radix_pass(ctx->ikeys2, ctx->ivals, ctx->ikeys, ctx->ivals2, n, 1, ctx->inst_hist,
                           ctx->inst_lookback, ctx->inst_tiles, ctx->err, s);
         order = ctx->ivals2;
     }
@@ -515,9 +519,10 @@ int force_pass(nb_ctx *ctx, Marks &mk) {
         launch_bbox_reduce(ctx->pos, n, ctx->bbox, s);
     }
     mk.mark(kMorton);
-    launch_morton_hist(ctx->pos, n, ctx->bbox, ctx->keys, ctx->sw.hist, s);
+    NB_TRY(clear_sort(n, ctx->sw, s), "radix sort");
+    launch_morton_hist(ctx->pos, n, ctx->bbox, ctx->keys, n > kSmallSort ? ctx->sw.hist : nullptr, s);
     mk.mark(kSort);
-    NB_TRY(launch_radix_sort(ctx->keys, ctx->vals, n, ctx->sw, ctx->err, s), "radix sort");
+    NB_TRY(launch_radix_sort(ctx->keys, ctx->keys, ctx->vals, n, ctx->sw, ctx->err, s), "radix sort");
     mk.mark(kGather);
     launch_gather_state(ctx->vals, n, ctx->pos, ctx->vel, ctx->id, ctx->pos2, ctx->vel2, ctx->id2, s);
     std::swap(ctx->pos, ctx->pos2);
@@ -613,9 +618,7 @@ int nb_create(const nb_config *cfg, nb_ctx **out) {
     }
     ctx->stream = ctx->own_stream;
     if (dev_alloc(&ctx->bbox, 1) != cudaSuccess || dev_alloc(&ctx->counts, 4) != cudaSuccess ||
-        dev_alloc(&ctx->err, 1) != cudaSuccess || dev_alloc(&ctx->sw.hist, 8 * 256) != cudaSuccess ||
-        dev_alloc(&ctx->sw.offsets, 8 * 256 + 8) != cudaSuccess || dev_alloc(&ctx->sw.tile_counter, 8) != cudaSuccess ||
-        dev_alloc(&ctx->tw.num_nodes, 1) != cudaSuccess) {
+        dev_alloc(&ctx->err, 1) != cudaSuccess || dev_alloc(&ctx->tw.num_nodes, 1) != cudaSuccess) {
         nb_destroy(ctx);
         return NB_ERR_OUT_OF_MEMORY;
     }
@@ -644,8 +647,7 @@ int nb_destroy(nb_ctx *ctx) {
     drop_graph(ctx);
     free_batch(ctx);
     free_buffers(ctx);
-    dev_free(ctx->bbox); dev_free(ctx->counts); dev_free(ctx->err); dev_free(ctx->sw.hist);
-    dev_free(ctx->sw.offsets); dev_free(ctx->sw.tile_counter); dev_free(ctx->tw.num_nodes); dev_free(ctx->acc64);
+    dev_free(ctx->bbox); dev_free(ctx->counts); dev_free(ctx->err); dev_free(ctx->tw.num_nodes); dev_free(ctx->acc64);
     dev_free(ctx->trav.stack); dev_free(ctx->trav.group_counter);
     if (ctx->host_scratch) cudaFreeHost(ctx->host_scratch);
     for (auto &ev: ctx->pending) ctx->event_pool.insert(ctx->event_pool.end(), ev.begin(), ev.end());
@@ -1070,7 +1072,7 @@ static int build_batch_tables(nb_ctx *ctx, int32_t count, const int64_t *sizes, 
     std::vector<int2> range((size_t) count);
     std::vector<int> group_first((size_t) count);
     std::vector<float> theta2((size_t) count);
-    std::vector<uint32_t> offsets(8 * 256 + 8, 0), hist(2 * 256, 0);
+    std::vector<uint32_t> hist(2 * 256, 0);
     ctx->inst_start.resize(count);
     ctx->inst_size.assign(sizes, sizes + count);
     int64_t start = 0, ngroups = 0;
@@ -1088,16 +1090,6 @@ static int build_batch_tables(nb_ctx *ctx, int32_t count, const int64_t *sizes, 
     const int64_t largest = count > 0 ? *std::max_element(sizes, sizes + count) : 1;
     ctx->inst_bbox_slices = (int) std::min<int64_t>(std::max<int64_t>((largest + 8191) / 8192, 1), 64);
     const int passes = count > 256 ? 2 : 1;
-    for (int p = 0; p < passes; ++p) {
-        uint32_t acc = 0;
-        bool trivial = false;
-        for (int d = 0; d < 256; ++d) {
-            offsets[p * 256 + d] = acc;
-            acc += hist[p * 256 + d];
-            if ((int64_t) hist[p * 256 + d] == n) trivial = true;
-        }
-        offsets[8 * 256 + p] = trivial ? 1u : 0u;
-    }
     const int64_t tiles = sort_tiles(n);
     if (n > ctx->batch_body_cap) {  // per-body buffers grow only
         dev_free(ctx->inst_of); dev_free(ctx->ikeys); dev_free(ctx->ikeys2); dev_free(ctx->ivals);
@@ -1130,7 +1122,7 @@ static int build_batch_tables(nb_ctx *ctx, int32_t count, const int64_t *sizes, 
         NB_TRY(dev_alloc(&ctx->groups, (size_t) ngroups), "alloc batch");
         ctx->batch_group_cap = ngroups;
     }
-    if (!ctx->inst_offsets) NB_TRY(dev_alloc(&ctx->inst_offsets, offsets.size()), "alloc batch");
+    if (!ctx->inst_hist) NB_TRY(dev_alloc(&ctx->inst_hist, hist.size()), "alloc batch");
     if (!ctx->inst_tiles) NB_TRY(dev_alloc(&ctx->inst_tiles, 8), "alloc batch");
     (void) tiles;
     int *group_first_dev = ctx->group_first;
@@ -1141,7 +1133,7 @@ static int build_batch_tables(nb_ctx *ctx, int32_t count, const int64_t *sizes, 
     NB_TRY(cudaMemcpyAsync(group_first_dev, group_first.data(), group_first.size() * sizeof(int), cudaMemcpyHostToDevice,
                            s), "copy");
     launch_fill_tables(ctx->inst_range, group_first_dev, count, ctx->inst_of, ctx->groups, s);
-    NB_TRY(cudaMemcpyAsync(ctx->inst_offsets, offsets.data(), offsets.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, s),
+    NB_TRY(cudaMemcpyAsync(ctx->inst_hist, hist.data(), hist.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, s),
            "copy");
     ctx->num_inst = count;
     ctx->ngroups = ngroups;

@@ -154,37 +154,48 @@ enum DeviceError : uint32_t {
 // bbox_morton.cu
 void launch_bbox_reset(BBoxAccum *acc, cudaStream_t s);
 void launch_bbox_reduce(const float4 *pos, int64_t n, BBoxAccum *acc, cudaStream_t s);
+// Codes, and their digit counts added to hist (skipped for hist == nullptr).
 void launch_morton_hist(const float4 *pos, int64_t n, const BBoxAccum *acc, uint64_t *codes, uint32_t *hist,
                         cudaStream_t s);
 
 // radix_sort.cu
-constexpr int kSortTileKeys = 2048;  // keys ranked per block (tile) of one one-sweep pass
+constexpr int kSortTileKeys = 4096;  // keys ranked per block (tile) of one one-sweep pass
 constexpr int kSortPasses = 8;       // 8-bit digits of the 64-bit keys
 struct SortWorkspace {
     uint64_t *keys_alt = nullptr;
     uint32_t *vals_alt = nullptr;
-    uint32_t *hist = nullptr;      // 8 x 256 digit counts, filled by launch_morton_hist
-    uint32_t *offsets = nullptr;   // 8 x 256 exclusive prefixes + 8 trivial-pass flags
-    uint32_t *lookback = nullptr;  // 8 x tiles x 256
-    uint32_t *tile_counter = nullptr;  // 8
+    // one block of memory, zero before the digit counts are taken (clear_sort):
+    uint32_t *hist = nullptr;          // 8 x 256 digit counts, filled by launch_morton_hist
+    uint32_t *tile_counter = nullptr;  // 8 (kSortHead words after hist's start: lookback)
+    uint32_t *lookback = nullptr;      // 8 x tiles x 256
     int64_t capacity = 0;
 };
 int64_t sort_tiles(int64_t n);
 size_t sort_lookback_words(int64_t n);
-// Sorts (keys, iota) by key; the sorted keys and slot indices end in keys/vals (ping-pong inside).
-// Returns the first error reported while queuing its memsets and launches (checked with
+constexpr int kSortHead = kSortPasses * 256 + 64;  // words before the look-back flags
+inline size_t sort_words(int64_t n) { return kSortHead + sort_lookback_words(n); }
+// Points a workspace's digit counts, tile tickets and look-back flags into `block` (sort_words(n) words).
+inline void place_sort(SortWorkspace &ws, uint32_t *block) {
+    ws.hist = block;
+    ws.tile_counter = block + kSortPasses * 256;
+    ws.lookback = block + kSortHead;
+}
+constexpr int64_t kSmallSort = 16384;  // largest key count sorted by one cluster (no histograms needed)
+cudaError_t clear_sort(int64_t n, SortWorkspace &ws, cudaStream_t s);
+// Sorts (src, iota) by key; the sorted keys and slot indices end in keys/vals (ping-pong inside; src
+// may be keys). Above kSmallSort keys the workspace holds the keys' digit counts and was cleared
+// before they were taken. Returns the first error reported while queuing its launches (checked with
 // cudaPeekAtLastError, which clears nothing).
-cudaError_t launch_radix_sort(uint64_t *keys, uint32_t *vals, int64_t n, SortWorkspace &ws, uint32_t *err,
-                              cudaStream_t s);
+cudaError_t launch_radix_sort(const uint64_t *src, uint64_t *keys, uint32_t *vals, int64_t n, SortWorkspace &ws,
+                              uint32_t *err, cudaStream_t s);
 // Self-test of the bounded look-back wait: one pass that can never complete its look-back runs
 // with the given wait limit; the error word it leaves is returned (kErrLookbackTimeout expected).
 cudaError_t lookback_timeout_selftest(unsigned long long wait_limit_ns, uint32_t *err_word);
-// One stable one-sweep pass on digit `pass` (bits 8*pass .. 8*pass+7) of the keys. offsets holds
-// the exclusive digit prefixes at [pass*256 + d] and a trivial-pass flag at [8*256 + pass];
-// lookback (pass x tiles x 256 words) and tile_counter[pass] must be zero. Pass 0 ignores vals_in
+// One stable one-sweep pass on digit `pass` (bits 8*pass .. 8*pass+7) of the keys. hist holds the
+// digit counts at [pass*256 + d]; lookback (pass x tiles x 256 words) and tile_counter[pass] must be zero. Pass 0 ignores vals_in
 // and emits the input positions as values.
 void launch_radix_pass(const uint64_t *keys_in, const uint32_t *vals_in, uint64_t *keys_out, uint32_t *vals_out,
-                       int64_t n, int pass, const uint32_t *offsets, uint32_t *lookback, uint32_t *tile_counter,
+                       int64_t n, int pass, const uint32_t *hist, uint32_t *lookback, uint32_t *tile_counter,
                        uint32_t *err, cudaStream_t s);
 
 // Several independent instances laid out back to back in one body array (device pointers).

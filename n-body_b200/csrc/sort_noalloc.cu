@@ -34,16 +34,12 @@ constexpr int64_t kMaxTiles = (kNoAllocMaxKeys + kSortTileKeys - 1) / kSortTileK
 constexpr size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 constexpr size_t kOffKeys = 0;
 constexpr size_t kOffVals = align256(kOffKeys + sizeof(uint64_t) * kNoAllocMaxKeys);
-constexpr size_t kOffHist = align256(kOffVals + sizeof(uint32_t) * kNoAllocMaxKeys);
-constexpr size_t kOffOffsets = align256(kOffHist + sizeof(uint32_t) * kSortPasses * 256);
-constexpr size_t kOffLookback = align256(kOffOffsets + sizeof(uint32_t) * (kSortPasses * 256 + kSortPasses));
+constexpr size_t kOffErr = align256(kOffVals + sizeof(uint32_t) * kNoAllocMaxKeys);
+// digit counts, tile tickets and look-back flags (place_sort), right behind the status word: one
+// clear covers both
+constexpr size_t kOffSort = kOffErr + 256;
 constexpr size_t kLookbackWords = (size_t) kSortPasses * kMaxTiles * 256;
-constexpr size_t kOffTiles = align256(kOffLookback + sizeof(uint32_t) * kLookbackWords);
-constexpr size_t kOffErr = align256(kOffTiles + sizeof(uint32_t) * kSortPasses);
-constexpr size_t kNoAllocScratchBytes = align256(kOffErr + sizeof(uint32_t));
-// The sort's launcher clears sort_lookback_words(n) look-back words: at the largest n accepted they
-// must fit before the tile tickets.
-static_assert(kOffLookback + sizeof(uint32_t) * kLookbackWords <= kOffTiles, "look-back region overlaps");
+constexpr size_t kNoAllocScratchBytes = align256(kOffSort + sizeof(uint32_t) * (kSortHead + kLookbackWords));
 
 static __device__ __align__(256) unsigned char g_sort_scratch[kNoAllocScratchBytes];
 
@@ -104,25 +100,20 @@ extern "C" int nb_sort_codes_noalloc(const uint64_t *d_codes, uint64_t *d_sorted
     SortWorkspace ws;
     ws.keys_alt = (uint64_t *) (base + kOffKeys);
     ws.vals_alt = (uint32_t *) (base + kOffVals);
-    ws.hist = (uint32_t *) (base + kOffHist);
-    ws.offsets = (uint32_t *) (base + kOffOffsets);
-    ws.lookback = (uint32_t *) (base + kOffLookback);
-    ws.tile_counter = (uint32_t *) (base + kOffTiles);
+    place_sort(ws, (uint32_t *) (base + kOffSort));
     ws.capacity = kNoAllocMaxKeys;
     uint32_t *err = (uint32_t *) (base + kOffErr);
 
-    // The scratch keeps the previous call's contents: clear what must start at zero.
-    if (cudaMemsetAsync(ws.hist, 0, sizeof(uint32_t) * kSortPasses * 256, s) != cudaSuccess) return NB_ERR_CUDA;
-    if (cudaMemsetAsync(err, 0, sizeof(uint32_t), s) != cudaSuccess) return NB_ERR_CUDA;
-    if (cudaMemcpyAsync(d_sorted_codes, d_codes, (size_t) n * sizeof(uint64_t), cudaMemcpyDeviceToDevice, s) !=
-        cudaSuccess)
-        return NB_ERR_CUDA;
-    const int64_t blocks = std::min<int64_t>((n + 256 * 8 - 1) / (256 * 8), (int64_t) current_sm_count() * 4);
-    digit_hist_kernel<<<(unsigned) std::max<int64_t>(blocks, 1), 256, 0, s>>>(d_codes, n, ws.hist);
-    if (cudaPeekAtLastError() != cudaSuccess) return NB_ERR_CUDA;
-    // Sorts in place in (d_sorted_codes, d_sorted_ids) with the scratch as the other buffer; the
-    // launcher clears the look-back flags and tile tickets itself.
-    if (launch_radix_sort(d_sorted_codes, d_sorted_ids, n, ws, err, s) != cudaSuccess) return NB_ERR_CUDA;
+    if (n > kSmallSort) {
+        // The scratch keeps the previous call's contents: clear what must start at zero.
+        if (cudaMemsetAsync(err, 0, 256 + sizeof(uint32_t) * sort_words(n), s) != cudaSuccess) return NB_ERR_CUDA;
+        const int64_t blocks = std::min<int64_t>((n + 256 * 8 - 1) / (256 * 8), (int64_t) current_sm_count() * 4);
+        digit_hist_kernel<<<(unsigned) std::max<int64_t>(blocks, 1), 256, 0, s>>>(d_codes, n, ws.hist);
+        if (cudaPeekAtLastError() != cudaSuccess) return NB_ERR_CUDA;
+    }
+    // Sorts into (d_sorted_codes, d_sorted_ids) with the scratch as the other buffer.
+    if (launch_radix_sort(d_codes, d_sorted_codes, d_sorted_ids, n, ws, err, s) != cudaSuccess) return NB_ERR_CUDA;
+    if (n <= kSmallSort) return cudaStreamSynchronize(s) == cudaSuccess ? NB_OK : NB_ERR_CUDA;  // no waits to report
     uint32_t e = 0;
     if (cudaMemcpyAsync(&e, err, sizeof(uint32_t), cudaMemcpyDeviceToHost, s) != cudaSuccess) return NB_ERR_CUDA;
     if (cudaStreamSynchronize(s) != cudaSuccess) return NB_ERR_CUDA;
