@@ -271,7 +271,6 @@ void free_buffers(nb_ctx *ctx) {
     dev_free(ctx->tw.topo); dev_free(ctx->tw.parent); dev_free(ctx->tw.flags); dev_free(ctx->tw.visit);
     dev_free(ctx->tw.slot); dev_free(ctx->tw.chain);
     dev_free(ctx->tw.start); dev_free(ctx->tw.pre_base); dev_free(ctx->tw.scan_part);
-    dev_free(ctx->tw.leaf_parents); dev_free(ctx->tw.leaf_parents_count);
     dev_free(ctx->nodes.mac); dev_free(ctx->nodes.link); dev_free(ctx->nodes.pay);
     ctx->nodes.capacity = 0;
     ctx->cap = 0;
@@ -299,12 +298,10 @@ int ensure_capacity(nb_ctx *ctx, int64_t n) {
     ctx->sw.capacity = c;
     NB_TRY(dev_alloc(&ctx->tw.topo, c), "alloc tree");
     NB_TRY(dev_alloc(&ctx->tw.parent, c), "alloc tree");
-    NB_TRY(dev_alloc(&ctx->tw.flags, c), "alloc tree");
+    NB_TRY(dev_alloc(&ctx->tw.flags, c + 8), "alloc tree");
     NB_TRY(dev_alloc(&ctx->tw.visit, c), "alloc tree");
     NB_TRY(dev_alloc(&ctx->tw.slot, 4 * slots), "alloc summaries");
     NB_TRY(dev_alloc(&ctx->tw.chain, c), "alloc tree");
-    NB_TRY(dev_alloc(&ctx->tw.leaf_parents, c), "alloc tree");
-    NB_TRY(dev_alloc(&ctx->tw.leaf_parents_count, 1), "alloc tree");
     NB_TRY(dev_alloc(&ctx->tw.start, c + 1), "alloc tree");
     NB_TRY(dev_alloc(&ctx->tw.pre_base, c + 1), "alloc tree");
     NB_TRY(dev_alloc(&ctx->tw.scan_part, build_scan_tiles(c)), "alloc tree");
@@ -381,10 +378,8 @@ void collect_times(nb_ctx *ctx) {
 int64_t launches_per_pass(const nb_ctx *ctx, bool with_bbox, bool with_drift) {
     if (ctx->cfg.solver == NB_SOLVER_NAIVE) return 1 + (with_drift ? 1 : 0);
     // the dual path adds loadBalancedBreak to the same pipeline
-    // morton(1) + sort (8 passes, or 1 kernel) + gather(1) + karras(1) + scans(3) + summarize(1)
-    // + root-leaf(1) + traverse(1)
-    int64_t k = 1 + (ctx->n > kSmallSort ? 8 : 1) + 1 + 1 + 3 + 1 + 1 + 1;
-    if (ctx->n <= 1) k -= 5;  // no Karras internal nodes
+    // morton(1) + sort (8 passes, or 1 kernel) + gather(1) + build + traverse(1)
+    int64_t k = 1 + (ctx->n > kSmallSort ? 8 : 1) + 1 + build_launches(ctx->n) + 1;
     if (ctx->cfg.solver == NB_SOLVER_DUAL_LINEAR_BVH) k += 2;  // loadBalancedBreak and the near-field kernel
     return k + (with_bbox ? 1 : 0) + (with_drift ? 1 : 0);
 }
@@ -470,7 +465,8 @@ int force_pass_batch(nb_ctx *ctx, Marks &mk) {
     }
     launch_compose(order, n, ctx->vals, ctx->keys, ctx->sw.vals_alt, ctx->sw.keys_alt, s);
     mk.mark(kGather);
-    launch_gather_state(ctx->sw.vals_alt, n, ctx->pos, ctx->vel, ctx->id, ctx->pos2, ctx->vel2, ctx->id2, s);
+    launch_gather_state(ctx->sw.vals_alt, n, ctx->pos, ctx->vel, ctx->id, ctx->pos2, ctx->vel2, ctx->id2,
+                        ctx->tw.start, s);
     std::swap(ctx->pos, ctx->pos2);
     std::swap(ctx->vel, ctx->vel2);
     std::swap(ctx->id, ctx->id2);
@@ -499,7 +495,7 @@ int force_pass_batch(nb_ctx *ctx, Marks &mk) {
 int force_pass(nb_ctx *ctx, Marks &mk) {
     const int64_t n = ctx->n;
     cudaStream_t s = ctx->stream;
-    cudaMemsetAsync(ctx->counts, 0, 4 * sizeof(unsigned long long), s);
+    cudaMemsetAsync(ctx->counts, 0, 5 * sizeof(unsigned long long), s);
     ctx->acc_is_dual = false;
     const bool need_bbox = !ctx->bbox_valid;
     mk.mark(kBBox);
@@ -524,7 +520,8 @@ int force_pass(nb_ctx *ctx, Marks &mk) {
     mk.mark(kSort);
     NB_TRY(launch_radix_sort(ctx->keys, ctx->keys, ctx->vals, n, ctx->sw, ctx->err, s), "radix sort");
     mk.mark(kGather);
-    launch_gather_state(ctx->vals, n, ctx->pos, ctx->vel, ctx->id, ctx->pos2, ctx->vel2, ctx->id2, s);
+    launch_gather_state(ctx->vals, n, ctx->pos, ctx->vel, ctx->id, ctx->pos2, ctx->vel2, ctx->id2,
+                        ctx->tw.start, s);
     std::swap(ctx->pos, ctx->pos2);
     std::swap(ctx->vel, ctx->vel2);
     std::swap(ctx->id, ctx->id2);
@@ -617,7 +614,7 @@ int nb_create(const nb_config *cfg, nb_ctx **out) {
         return NB_ERR_CUDA;
     }
     ctx->stream = ctx->own_stream;
-    if (dev_alloc(&ctx->bbox, 1) != cudaSuccess || dev_alloc(&ctx->counts, 4) != cudaSuccess ||
+    if (dev_alloc(&ctx->bbox, 1) != cudaSuccess || dev_alloc(&ctx->counts, 5) != cudaSuccess ||
         dev_alloc(&ctx->err, 1) != cudaSuccess || dev_alloc(&ctx->tw.num_nodes, 1) != cudaSuccess) {
         nb_destroy(ctx);
         return NB_ERR_OUT_OF_MEMORY;
@@ -627,8 +624,9 @@ int nb_create(const nb_config *cfg, nb_ctx **out) {
         return NB_ERR_OUT_OF_MEMORY;
     }
     ctx->trav.warps = traverse_resident_warps(cfg->device);
-    if (dev_alloc(&ctx->trav.stack, (size_t) ctx->trav.warps * kWarpScratch) != cudaSuccess ||
-        dev_alloc(&ctx->trav.group_counter, 1) != cudaSuccess) {
+    // the traversal's work counter sits behind the interaction counts: one clear per pass covers both
+    ctx->trav.group_counter = (unsigned *) (ctx->counts + 4);
+    if (dev_alloc(&ctx->trav.stack, (size_t) ctx->trav.warps * kWarpScratch) != cudaSuccess) {
         nb_destroy(ctx);
         return NB_ERR_OUT_OF_MEMORY;
     }
@@ -648,7 +646,7 @@ int nb_destroy(nb_ctx *ctx) {
     free_batch(ctx);
     free_buffers(ctx);
     dev_free(ctx->bbox); dev_free(ctx->counts); dev_free(ctx->err); dev_free(ctx->tw.num_nodes); dev_free(ctx->acc64);
-    dev_free(ctx->trav.stack); dev_free(ctx->trav.group_counter);
+    dev_free(ctx->trav.stack);
     if (ctx->host_scratch) cudaFreeHost(ctx->host_scratch);
     for (auto &ev: ctx->pending) ctx->event_pool.insert(ctx->event_pool.end(), ev.begin(), ev.end());
     for (auto e: ctx->event_pool) cudaEventDestroy(e);

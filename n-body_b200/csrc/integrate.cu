@@ -6,7 +6,8 @@
 // step's Morton quantisation needs no separate pass over the bodies.
 //
 // Bodies live in the order of the last Morton sort; gather_state permutes positions, velocities
-// and input ids after each sort so the traversal reads its targets and leaf bodies contiguously.
+// and input ids after each sort so the traversal reads its targets and leaf bodies contiguously (and
+// clears the node counts that the build adds to).
 // All kernels here are HBM-bound streaming kernels.
 #include <cfloat>
 
@@ -26,8 +27,10 @@ __global__ void __launch_bounds__(kThreads) gather_state_kernel(const uint32_t *
                                                                  const uint32_t *__restrict__ id,
                                                                  float4 *__restrict__ pos_out,
                                                                  float4 *__restrict__ vel_out,
-                                                                 uint32_t *__restrict__ id_out) {
+                                                                 uint32_t *__restrict__ id_out,
+                                                                 int *__restrict__ start) {
     const int64_t k = (int64_t) blockIdx.x * blockDim.x + threadIdx.x;
+    if (k <= n) start[k] = 0;  // n + 1 node counts of the build that follows
     if (k >= n) return;
     const uint32_t src = perm[k];
     if (src >= (uint64_t) n) return;  // defensive: a failed sort never makes this read out of bounds
@@ -105,9 +108,9 @@ __global__ void __launch_bounds__(kThreads) kick_drift_kernel(float4 *__restrict
 }  // namespace
 
 void launch_gather_state(const uint32_t *perm, int64_t n, const float4 *pos, const float4 *vel, const uint32_t *id,
-                         float4 *pos_out, float4 *vel_out, uint32_t *id_out, cudaStream_t s) {
+                         float4 *pos_out, float4 *vel_out, uint32_t *id_out, int *start, cudaStream_t s) {
     if (n <= 0) return;
-    gather_state_kernel<<<blocks_for(n), kThreads, 0, s>>>(perm, n, pos, vel, id, pos_out, vel_out, id_out);
+    gather_state_kernel<<<blocks_for(n + 1), kThreads, 0, s>>>(perm, n, pos, vel, id, pos_out, vel_out, id_out, start);
 }
 
 void launch_scatter_by_id(const uint32_t *id, int64_t n, const float4 *src, float4 *dst, cudaStream_t s) {

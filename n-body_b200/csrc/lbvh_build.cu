@@ -17,15 +17,16 @@
 //                     and the number of final nodes starting at each body position
 //   scan kernels      exclusive prefix over body positions of those counts: the preorder index of
 //                     the final leaf starting at each position
-//   summarize_kernel  one thread per final internal node with leaf children: sequential leaf
-//                     summaries over the leaf's bodies, then an atomic climb in which the second
-//                     child to arrive summarises the parent (CenterOfMassSummary.h:30-55,
+//   summarize_kernel  one block per kClimbNodes Karras nodes, one thread per final internal node with
+//                     leaf children: sequential leaf summaries over the leaf's bodies, then a climb in
+//                     which the second child to arrive summarises the parent (CenterOfMassSummary.h:30-55,
 //                     BoundingBoxSummary.h:30-68, MultipoleMassSummary.h:37-97; the leaf moment
 //                     sum follows libstdc++'s 4-way std::transform_reduce). All float operations
 //                     are single IEEE operations in the reference's order, so summaries are
-//                     bit-identical to the CPU restatement. Every node's record (the arrays the
-//                     traversal reads: MAC data, links, payload) is written by the thread that
-//                     finishes the node, at the node's preorder index. That index is closed-form:
+//                     bit-identical to the CPU restatement. The records (the arrays the traversal
+//                     reads: MAC data, links, payload) of the nodes that a block finishes alone are
+//                     written by its threads together, others by the thread that finishes the node,
+//                     at the node's preorder index. That index is closed-form:
 //                     for a node whose range starts at body f, the final nodes before it in
 //                     preorder are those starting before f and, among the internal nodes starting
 //                     at f (a chain of left children), the larger ones; a leaf starting at f comes
@@ -105,15 +106,17 @@ __global__ void __launch_bounds__(kThreads) karras_kernel(const uint64_t *__rest
         const bool rleaf = rc < 0 || !range_splittable(codes, inst_of, leaf, gamma + 1, last);
         if (lleaf) atomicAdd(tw.start + first, 1);
         if (rleaf) atomicAdd(tw.start + gamma + 1, 1);
-        if (lleaf || rleaf) tw.leaf_parents[atomicAdd(tw.leaf_parents_count, 1)] = i;
         f |= (uint8_t) ((lleaf ? kLeftLeaf : 0) | (rleaf ? kRightLeaf : 0));
     }
     tw.flags[i] = f;
 }
 
-// Exclusive prefix over positions 0..n of the number of final nodes starting at each position,
-// in three steps: tile totals, a prefix over the tiles (one block), and the per-tile scan.
+// Exclusive prefix over positions 0..n of the number of final nodes starting at each position. A
+// block of scan_apply finds the sum before its tile itself: from the positions, up to kScanDirect
+// tiles (one kernel); from the tiles' totals, up to kScanParts tiles (scan_tiles first); beyond that the
+// totals' prefix is taken by one block in between, so that the work stays linear.
 constexpr int kScanTile = 2048;
+constexpr int kScanDirect = 8, kScanParts = 4096;
 
 __device__ __forceinline__ int starts_at(const int *__restrict__ start, int64_t b) {
     const int w = start[b];
@@ -165,10 +168,35 @@ __global__ void __launch_bounds__(1024) scan_parts_kernel(int *__restrict__ part
     if (threadIdx.x == 0) *total = carry;
 }
 
+// The block's sum of v over its threads (every thread gets it).
+__device__ __forceinline__ int block_sum(int v, int *red) {
+    v = __reduce_add_sync(0xffffffffu, v);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+    __syncthreads();
+    int t = 0;
+#pragma unroll
+    for (int w = 0; w < kThreads / 32; ++w) t += red[w];
+    return t;
+}
+
 // Writes pre_base[f] = (final nodes starting before f) + (final internal nodes starting at f): the
 // preorder index of the final leaf starting at f, one past the smallest internal node starting there.
+// `before` says where the sum before the tile comes from: kFromStart, kFromTotals or kFromPrefix.
+enum : int { kFromStart = 0, kFromTotals = 1, kFromPrefix = 2 };
 __global__ void __launch_bounds__(kThreads) scan_apply_kernel(const int *__restrict__ start, int64_t m,
-                                                              const int *__restrict__ part, int *__restrict__ pre_base) {
+                                                              const int *__restrict__ part, int before,
+                                                              int *__restrict__ pre_base, int *__restrict__ total) {
+    __shared__ int red[kThreads / 32];
+    int prefix = 0;
+    if (before == kFromPrefix) {
+        prefix = part[blockIdx.x];
+    } else {
+        const int64_t count = before == kFromStart ? (int64_t) blockIdx.x * kScanTile : blockIdx.x;
+        int sum = 0;
+#pragma unroll 4
+        for (int64_t k = threadIdx.x; k < count; k += kThreads) sum += before == kFromStart ? starts_at(start, k) : part[k];
+        prefix = block_sum(sum, red);
+    }
     constexpr int kPer = kScanTile / kThreads;  // consecutive positions per thread
     __shared__ int warp_sum[kThreads / 32];
     const int64_t base = (int64_t) blockIdx.x * kScanTile + (int64_t) threadIdx.x * kPer;
@@ -189,13 +217,15 @@ __global__ void __launch_bounds__(kThreads) scan_apply_kernel(const int *__restr
     }
     if (lane == 31) warp_sum[warp] = incl;
     __syncthreads();
-    int run = part[blockIdx.x] + incl - sum;
+    int run = prefix + incl - sum;
     for (int w = 0; w < warp; ++w) run += warp_sum[w];
 #pragma unroll
     for (int k = 0; k < kPer; ++k) {
         if (base + k < m) pre_base[base + k] = run + (w[k] >> 1);
         run += v[k];
     }
+    // the last position's sum is the number of final nodes
+    if (before != kFromPrefix && base < m && base + kPer >= m) *total = run;
 }
 
 // Preorder index of a final node whose range starts at body f: after the final nodes starting
@@ -311,8 +341,12 @@ template<int ORDER>
 __device__ Summ<ORDER> leaf_summary(const float4 *__restrict__ bodies, int b, int e /* inclusive */) {
     Summ<ORDER> s;
     float M = 0.f, cx = 0.f, cy = 0.f, cz = 0.f;
+    float mn[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, mx[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
+#pragma unroll 4
     for (int i = b; i <= e; ++i) {
         const float4 p = bodies[i];
+        mn[0] = gmin(p.x, mn[0]); mn[1] = gmin(p.y, mn[1]); mn[2] = gmin(p.z, mn[2]);
+        mx[0] = gmax(p.x, mx[0]); mx[1] = gmax(p.y, mx[1]); mx[2] = gmax(p.z, mx[2]);
         M = fadd(M, p.w);
         cx = fadd(cx, fmul(p.w, p.x));
         cy = fadd(cy, fmul(p.w, p.y));
@@ -355,12 +389,6 @@ __device__ Summ<ORDER> leaf_summary(const float4 *__restrict__ bodies, int b, in
 #pragma unroll
             for (int k = 0; k < 10; ++k) s.q3[k] = acc[6 + k];
         }
-    }
-    float mn[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, mx[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
-    for (int i = b; i <= e; ++i) {
-        const float4 p = bodies[i];
-        mn[0] = gmin(p.x, mn[0]); mn[1] = gmin(p.y, mn[1]); mn[2] = gmin(p.z, mn[2]);
-        mx[0] = gmax(p.x, mx[0]); mx[1] = gmax(p.y, mx[1]); mx[2] = gmax(p.z, mx[2]);
     }
 #pragma unroll
     for (int k = 0; k < 3; ++k) { s.bmin[k] = mn[k]; s.bmax[k] = mx[k]; }
@@ -611,30 +639,60 @@ __device__ __forceinline__ Summ<ORDER> combine(const TreeWorkspace &tw, const Su
                                                                               : internal_summary<ORDER>(l, r);
 }
 
-// Final internal node i's final-leaf children: leaf summaries and records, then the climb. A node
-// whose children are both final leaves is finished at once, without an arrival. The topology of
-// the next node up is loaded while the current level computes, so a level waits for its arrival
-// and the sibling's summary only.
+// One block per kClimbNodes Karras nodes. All descendants of a node that covers bodies [first, last] have
+// Karras indices in [first, last], so a node whose range lies in the block's index range is climbed
+// to by this block's threads alone: its arrivals are counted in shared memory and need block-scope
+// ordering only, a few hundred cycles instead of the device-scope arrival's round trips to L2.
+constexpr int kClimbNodes = 1024;
+constexpr int kClimbThreads = 128;
+static_assert(kClimbNodes == 8 * kClimbThreads, "eight node flags per thread");
+
+struct ClimbSmem {
+    int visit[kClimbNodes];
+    uint16_t list[2][kClimbNodes];  // the block's final internal nodes: those with leaf children, all of them
+    int count[2];
+};
+
+__device__ __forceinline__ bool in_block(int4 tp) {
+    const int lo = blockIdx.x * kClimbNodes;
+    return tp.z >= lo && tp.w < lo + kClimbNodes;
+}
+
+// Final internal node i's final-leaf children: leaf summaries, then the climb. A node whose children
+// are both final leaves is finished at once, without an arrival. The topology of the next node up is
+// loaded while the current level computes. Records of nodes beyond the block's own are written on
+// the way, after the arrival at the parent.
 template<int ORDER, class Records>
 __device__ void summarize_from(const float4 *__restrict__ bodies, int n, const TreeWorkspace &tw, uint32_t *err,
-                               const Records &rec, int i) {
+                               const Records &rec, ClimbSmem &S, int i) {
+    const int lo = blockIdx.x * kClimbNodes;
     int4 tp = tw.topo[i];  // (left child, right child, first body, last body) of the node p below
     uint8_t fl = tw.flags[i];
     int par = tw.parent[i];  // not written for the root, and read only below a non-root node
     const int gamma = tp.x >= 0 ? tp.x : ~tp.x;  // the left child's last body
     Summ<ORDER> mine;
     int from, p, chain_from;  // the finished child and its chain (-1: a leaf), the node above it
+    bool pending = false;     // the finished child's record is to be written here:
+    int pre = 0, first = 0, last = 0, right_pre = 0;  // its preorder index, range, right child's index
     if ((fl & kLeftLeaf) && (fl & kRightLeaf)) {
         const Summ<ORDER> l = leaf_summary<ORDER>(bodies, tp.z, gamma);
         const Summ<ORDER> r = leaf_summary<ORDER>(bodies, gamma + 1, tp.w);
-        rec.leaf(preorder_leaf(tw, tp.z), l, tp.z, gamma, err);
-        const int right_pre = preorder_leaf(tw, gamma + 1);
-        rec.leaf(right_pre, r, gamma + 1, tp.w, err);
+        store_slot<ORDER>(tw, slot_of(tp.x, n), l);
+        store_slot<ORDER>(tw, slot_of(tp.y, n), r);
         mine = combine<ORDER>(tw, l, r, tp.z, tp.w);
         store_slot<ORDER>(tw, i, mine);
         tw.chain[i] = 0;
-        rec.internal(preorder_internal(tw, tp.z, 0), mine, tp.z, tp.w, right_pre, err);
-        if (i == 0) return;
+        if (!in_block(tp)) {
+            pending = true;
+            right_pre = preorder_leaf(tw, gamma + 1);
+            pre = preorder_internal(tw, tp.z, 0);
+            first = tp.z;
+            last = tp.w;
+        }
+        if (i == 0) {
+            if (pending) rec.internal(pre, mine, first, last, right_pre, err);
+            return;
+        }
         from = i;
         chain_from = 0;
         p = par;
@@ -647,11 +705,9 @@ __device__ void summarize_from(const float4 *__restrict__ bodies, int n, const T
         par = tw.parent[p];
     } else {
         const bool left = (fl & kLeftLeaf) != 0;  // exactly one child is a final leaf
-        const int b = left ? tp.z : gamma + 1, e = left ? gamma : tp.w;
-        mine = leaf_summary<ORDER>(bodies, b, e);
+        mine = leaf_summary<ORDER>(bodies, left ? tp.z : gamma + 1, left ? gamma : tp.w);
         from = left ? tp.x : tp.y;
         store_slot<ORDER>(tw, slot_of(from, n), mine);
-        rec.leaf(preorder_leaf(tw, b), mine, b, e, err);
         chain_from = -1;
         p = i;
     }
@@ -660,34 +716,53 @@ __device__ void summarize_from(const float4 *__restrict__ bodies, int n, const T
             atomicOr(err, (uint32_t) kErrTreeDepth);
             return;
         }
-        if (arrive_acq_rel(&tw.visit[p]) == 0) return;  // the sibling's thread finishes p
+        const bool own = in_block(tp);
+        bool second;
+        if (own) {
+            __threadfence_block();
+            second = atomicAdd(&S.visit[p - lo], 1) != 0;
+            __threadfence_block();
+        } else {
+            second = arrive_acq_rel(&tw.visit[p]) != 0;
+        }
         const int lc = tp.x, rc = tp.y;
         const bool from_left = (lc == from);
         const bool lfin = (fl & kLeftLeaf) != 0, rfin = (fl & kRightLeaf) != 0;
         const int sib = from_left ? rc : lc;
-        const Summ<ORDER> other = load_slot<ORDER>(tw, slot_of(sib, n));
-        const int sib_chain = (from_left ? rfin : lfin) ? -1 : __ldcg(tw.chain + sib);
+        Summ<ORDER> other;
+        int sib_chain = -1, npar = -1;
         int4 ntp = make_int4(0, 0, 0, 0);
         uint8_t nfl = 0;
-        int npar = -1;
-        if (p != 0 && par >= 0 && par < n - 1) {
-            ntp = tw.topo[par];
-            nfl = tw.flags[par];
-            npar = tw.parent[par];
+        if (second) {
+            other = load_slot<ORDER>(tw, slot_of(sib, n));
+            if (!(from_left ? rfin : lfin)) sib_chain = __ldcg(tw.chain + sib);
+            if (p != 0 && par >= 0 && par < n - 1) {
+                ntp = tw.topo[par];
+                nfl = tw.flags[par];
+                npar = tw.parent[par];
+            }
         }
-        const Summ<ORDER> up = from_left ? combine<ORDER>(tw, mine, other, tp.z, tp.w)
-                                         : combine<ORDER>(tw, other, mine, tp.z, tp.w);
-        store_slot<ORDER>(tw, p, up);
+        if (pending) rec.internal(pre, mine, first, last, right_pre, err);
+        if (!second) return;  // the sibling's thread finishes p
+        mine = from_left ? combine<ORDER>(tw, mine, other, tp.z, tp.w) : combine<ORDER>(tw, other, mine, tp.z, tp.w);
+        store_slot<ORDER>(tw, p, mine);
         // final internal nodes below p that share its first body: its left child's chain
         const int lchain = lfin ? -1 : (from_left ? chain_from : sib_chain);
         const int rchain = rfin ? -1 : (from_left ? sib_chain : chain_from);
         const int ch = lchain + 1;
         tw.chain[p] = ch;
-        const int rfirst = (lc >= 0 ? lc : ~lc) + 1;
-        const int right_pre = rfin ? preorder_leaf(tw, rfirst) : preorder_internal(tw, rfirst, rchain);
-        rec.internal(preorder_internal(tw, tp.z, ch), up, tp.z, tp.w, right_pre, err);
-        if (p == 0) return;
-        mine = up;
+        pending = !own;
+        if (pending) {
+            const int rfirst = (lc >= 0 ? lc : ~lc) + 1;
+            right_pre = rfin ? preorder_leaf(tw, rfirst) : preorder_internal(tw, rfirst, rchain);
+            pre = preorder_internal(tw, tp.z, ch);
+            first = tp.z;
+            last = tp.w;
+        }
+        if (p == 0) {
+            if (pending) rec.internal(pre, mine, first, last, right_pre, err);
+            return;
+        }
         chain_from = ch;
         from = p;
         p = par;
@@ -697,61 +772,92 @@ __device__ void summarize_from(const float4 *__restrict__ bodies, int n, const T
     }
 }
 
-// One thread per final internal node with leaf children (the compact list karras_kernel built), on
-// a grid of a few waves at most.
+// Records of the block's final internal node i, if the block finished it, and of its final-leaf children.
 template<int ORDER, class Records>
-__global__ void __launch_bounds__(kThreads) summarize_kernel(const float4 *__restrict__ bodies, int n, TreeWorkspace tw,
-                                                             uint32_t *err, Records rec) {
-    const int count = *tw.leaf_parents_count;
-    for (int idx = blockIdx.x * blockDim.x + threadIdx.x; idx < count; idx += gridDim.x * blockDim.x)
-        summarize_from<ORDER, Records>(bodies, n, tw, err, rec, tw.leaf_parents[idx]);
+__device__ void write_records(int n, const TreeWorkspace &tw, uint32_t *err, const Records &rec, int i) {
+    const int4 tp = tw.topo[i];
+    const uint8_t fl = tw.flags[i];
+    const int gamma = tp.x >= 0 ? tp.x : ~tp.x;
+    const bool lfin = (fl & kLeftLeaf) != 0, rfin = (fl & kRightLeaf) != 0;
+    if (in_block(tp)) {
+        const int right_pre = rfin ? preorder_leaf(tw, gamma + 1) : preorder_internal(tw, gamma + 1, __ldcg(tw.chain + tp.y));
+        rec.internal(preorder_internal(tw, tp.z, __ldcg(tw.chain + i)), load_slot<ORDER>(tw, i), tp.z, tp.w, right_pre, err);
+    }
+    if (lfin) rec.leaf(preorder_leaf(tw, tp.z), load_slot<ORDER>(tw, slot_of(tp.x, n)), tp.z, gamma, err);
+    if (rfin) rec.leaf(preorder_leaf(tw, gamma + 1), load_slot<ORDER>(tw, slot_of(tp.y, n)), gamma + 1, tp.w, err);
 }
 
-__global__ void root_leaf_dual_kernel(const float4 *__restrict__ bodies, int n, TreeWorkspace tw, DualNodes nodes,
-                                      float theta, uint32_t *err) {
-    if (n > 1 && (tw.flags[0] & kFinal)) return;
-    write_dual_record(nodes, 0, leaf_summary<3>(bodies, 0, n - 1), 0, n - 1, 0, n, theta, err);
-    *tw.num_nodes = 1;
+// Bound by latency: the climb's chain of levels, each an arrival, the sibling's summary and the IEEE divides
+// of the centre of mass. The records' threshold searches (several divides each) stay off the chain: the
+// block writes the records of its own nodes when its climbs are done, all threads at once. The block
+// lists its nodes with leaf children (then its final nodes) first, so that threads climb and do not idle
+// over the nodes in between. The whole tree is one leaf when n == 1, or when the root is not
+// splittable (n <= maxLeafSize or every code equal): the first block's first thread writes it.
+// Cold-cache times, before (device-scope arrivals at every level, records on the chain, a list of leaf
+// parents made by karras_kernel) and now: 1,023 bodies 66 and 47 us, 60,001 bodies (octupole) 160 and 141 us, 2^20
+// bodies 112 and 145 us with karras_kernel 73 and 46 us; four launches and clears fewer per build.
+template<int ORDER, class Records>
+__global__ void __launch_bounds__(kClimbThreads) summarize_kernel(const float4 *__restrict__ bodies, int n, TreeWorkspace tw,
+                                                                  uint32_t *err, Records rec) {
+    __shared__ ClimbSmem S;
+    if (n == 1 || !(tw.flags[0] & kFinal)) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) {
+            rec.leaf(0, leaf_summary<ORDER>(bodies, 0, n - 1), 0, n - 1, err);
+            *tw.num_nodes = 1;
+        }
+        return;
+    }
+    const int lo = blockIdx.x * kClimbNodes, count = min(kClimbNodes, n - 1 - lo);
+    if (threadIdx.x == 0) S.count[0] = S.count[1] = 0;
+    for (int k = threadIdx.x; k < count; k += kClimbThreads) S.visit[k] = 0;
+    __syncthreads();
+    {   // eight flags per thread in one load (the flags are padded to a multiple of eight)
+        const int k0 = 8 * threadIdx.x;
+        const uint64_t eight = k0 < count ? *reinterpret_cast<const uint64_t *>(tw.flags + lo + k0) : 0ull;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const unsigned fl = k0 + j < count ? (unsigned) (eight >> (8 * j)) & 255u : 0u;
+            if (fl & (kLeftLeaf | kRightLeaf)) S.list[0][atomicAdd(&S.count[0], 1)] = (uint16_t) (k0 + j);
+            if (fl & kFinal) S.list[1][atomicAdd(&S.count[1], 1)] = (uint16_t) (k0 + j);
+        }
+    }
+    __syncthreads();
+    for (int k = threadIdx.x; k < S.count[0]; k += kClimbThreads)
+        summarize_from<ORDER, Records>(bodies, n, tw, err, rec, S, lo + S.list[0][k]);
+    __syncthreads();
+    for (int k = threadIdx.x; k < S.count[1]; k += kClimbThreads)
+        write_records<ORDER, Records>(n, tw, err, rec, lo + S.list[1][k]);
 }
 
-// The whole tree is one leaf when n == 1, or when the root is not splittable (n <= maxLeafSize
-// or every code equal).
-template<int ORDER>
-__global__ void root_leaf_kernel(const float4 *__restrict__ bodies, int n, TreeWorkspace tw, float t,
-                                 NodeArrays nodes, uint32_t *err, BatchSegments seg) {
-    if (n > 1 && (tw.flags[0] & kFinal)) return;
-    write_record<ORDER>(nodes, 0, leaf_summary<ORDER>(bodies, 0, n - 1), node_theta2(seg, t, 0), 0, n, err);
-    register_root(seg, 0, 0, n - 1);
-    *tw.num_nodes = 1;
-}
+int summarize_blocks(int n) { return std::max(1, (n - 1 + kClimbNodes - 1) / kClimbNodes); }
 
-// Grid of the summary climb: enough threads for every possible leaf parent, capped at a few waves
-// (the kernel loops over the compact list).
-int summarize_blocks(int n) {
-    const int64_t need = ((int64_t) n - 1 + kThreads - 1) / kThreads;
-    const int64_t cap = (int64_t) current_sm_count() * 8;
-    return (int) std::max<int64_t>(1, std::min(need, cap));
-}
-
-// Karras topology, the final nodes per start position and their exclusive prefix (which also
-// gives the node count); the topology kernel also clears the climb's arrival counters.
+// Karras topology, the final nodes per start position (tw.start is zero on entry) and their
+// exclusive prefix (which also gives the node count); the topology kernel also clears the climb's
+// arrival counters.
 void launch_topology(const uint64_t *sorted_codes, const int *inst_of, int n, int leaf, TreeWorkspace &tw,
                      cudaStream_t s) {
     const int internal = n - 1;
     const int blocks = (internal + kThreads - 1) / kThreads;
     const int64_t m = (int64_t) n + 1;
     const int tiles = (int) build_scan_tiles(n);
-    cudaMemsetAsync(tw.start, 0, (size_t) m * sizeof(int), s);
-    cudaMemsetAsync(tw.leaf_parents_count, 0, sizeof(int), s);
     karras_kernel<<<blocks, kThreads, 0, s>>>(sorted_codes, inst_of, n, leaf, tw);
-    scan_tiles_kernel<<<tiles, kThreads, 0, s>>>(tw.start, m, tw.scan_part);
-    scan_parts_kernel<<<1, 1024, 0, s>>>(tw.scan_part, tiles, tw.num_nodes);
-    scan_apply_kernel<<<tiles, kThreads, 0, s>>>(tw.start, m, tw.scan_part, tw.pre_base);
+    if (tiles > kScanDirect) scan_tiles_kernel<<<tiles, kThreads, 0, s>>>(tw.start, m, tw.scan_part);
+    if (tiles > kScanParts) scan_parts_kernel<<<1, 1024, 0, s>>>(tw.scan_part, tiles, tw.num_nodes);
+    scan_apply_kernel<<<tiles, kThreads, 0, s>>>(tw.start, m, tw.scan_part,
+                                                 tiles > kScanParts    ? kFromPrefix
+                                                 : tiles > kScanDirect ? kFromTotals
+                                                                       : kFromStart,
+                                                 tw.pre_base, tw.num_nodes);
 }
 
 }  // namespace
 
 int64_t build_scan_tiles(int64_t n) { return (n + 1 + kScanTile - 1) / kScanTile; }
+
+int build_launches(int64_t n) {
+    const int64_t tiles = build_scan_tiles(n);
+    return n <= 1 ? 1 : 3 + (tiles > kScanDirect ? 1 : 0) + (tiles > kScanParts ? 1 : 0);
+}
 
 void launch_build_dual_tree(const uint64_t *sorted_codes, const float4 *bodies, int64_t n64, int leaf, float theta,
                             TreeWorkspace &tw, const DualNodes &nodes, uint32_t *err, cudaStream_t s) {
@@ -760,12 +866,9 @@ void launch_build_dual_tree(const uint64_t *sorted_codes, const float4 *bodies, 
         cudaMemsetAsync(tw.num_nodes, 0, sizeof(int), s);
         return;
     }
-    if (n > 1) {
-        launch_topology(sorted_codes, nullptr, n, leaf, tw, s);
-        summarize_kernel<3, DualRecords>
-            <<<summarize_blocks(n), kThreads, 0, s>>>(bodies, n, tw, err, DualRecords{nodes, theta});
-    }
-    root_leaf_dual_kernel<<<1, 1, 0, s>>>(bodies, n, tw, nodes, theta, err);
+    if (n > 1) launch_topology(sorted_codes, nullptr, n, leaf, tw, s);
+    summarize_kernel<3, DualRecords>
+        <<<summarize_blocks(n), kClimbThreads, 0, s>>>(bodies, n, tw, err, DualRecords{nodes, theta});
 }
 
 void launch_build_tree(const uint64_t *sorted_codes, const float4 *bodies, int64_t n64, int leaf, int order,
@@ -778,17 +881,12 @@ void launch_build_tree(const uint64_t *sorted_codes, const float4 *bodies, int64
     }
     const float t = theta * theta;  // the reference compares against theta * theta in float
     if (n > 1) launch_topology(sorted_codes, seg.inst_of, n, leaf, tw, s);
-    if (order == 1) {
-        if (n > 1)
-            summarize_kernel<1, BhRecords<1>>
-                <<<summarize_blocks(n), kThreads, 0, s>>>(bodies, n, tw, err, BhRecords<1>{nodes, t, seg});
-        root_leaf_kernel<1><<<1, 1, 0, s>>>(bodies, n, tw, t, nodes, err, seg);
-    } else {
-        if (n > 1)
-            summarize_kernel<2, BhRecords<2>>
-                <<<summarize_blocks(n), kThreads, 0, s>>>(bodies, n, tw, err, BhRecords<2>{nodes, t, seg});
-        root_leaf_kernel<2><<<1, 1, 0, s>>>(bodies, n, tw, t, nodes, err, seg);
-    }
+    if (order == 1)
+        summarize_kernel<1, BhRecords<1>>
+            <<<summarize_blocks(n), kClimbThreads, 0, s>>>(bodies, n, tw, err, BhRecords<1>{nodes, t, seg});
+    else
+        summarize_kernel<2, BhRecords<2>>
+            <<<summarize_blocks(n), kClimbThreads, 0, s>>>(bodies, n, tw, err, BhRecords<2>{nodes, t, seg});
 }
 
 }  // namespace nbg

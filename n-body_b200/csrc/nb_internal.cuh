@@ -222,9 +222,6 @@ struct TreeWorkspace {
     int *pre_base = nullptr;        // per body position (n + 1): preorder index of the final leaf starting there
                                     // (final nodes starting before it plus final internal nodes starting at it)
     int *scan_part = nullptr;       // per scan tile: its total, then its exclusive prefix
-    int *leaf_parents = nullptr;    // final internal nodes with at least one final-leaf child (n - 1),
-                                    // in no particular order; the count is leaf_parents_count[0]
-    int *leaf_parents_count = nullptr;
     int *num_nodes = nullptr;       // device scalar: final node count
     int64_t capacity = 0;
     // Precision option (0: off, the reference's FP32 operations everywhere): internal nodes of at
@@ -233,6 +230,9 @@ struct TreeWorkspace {
 };
 // Scan tiles of the preorder prefix over n + 1 body positions (sizes tw.scan_part).
 int64_t build_scan_tiles(int64_t n);
+// Kernel launches of one build over n bodies.
+int build_launches(int64_t n);
+// Both builds expect tw.start to be zero (launch_gather_state clears it).
 void launch_build_tree(const uint64_t *sorted_codes, const float4 *bodies, int64_t n, int leaf, int order, float theta,
                        TreeWorkspace &tw, const NodeArrays &nodes, uint32_t *err, cudaStream_t s,
                        const BatchSegments &seg = BatchSegments());
@@ -308,7 +308,7 @@ void launch_dual_traverse(const DualNodes &nodes, const int *num_nodes, const fl
 struct TraverseWorkspace {
     int2 *stack = nullptr;            // per resident warp: kTraverseStack entries of (node, target mask), then
                                       // the warp's leaf sums (kWarpScratch int2 in all)
-    unsigned *group_counter = nullptr;
+    unsigned *group_counter = nullptr;  // zero before each pass
     int64_t warps = 0;                // resident warps the stack memory was sized for
     int threads = 256;                // launch shape: threads per block (128 or 256)
     int slab = 64;                    // launch shape: partial-accept slab entries per warp (32 or 64)
@@ -345,7 +345,7 @@ void launch_direct_f64(const float4 *bodies, int64_t n, const float4 *targets, i
 
 // integrate.cu
 void launch_gather_state(const uint32_t *perm, int64_t n, const float4 *pos, const float4 *vel, const uint32_t *id,
-                         float4 *pos_out, float4 *vel_out, uint32_t *id_out, cudaStream_t s);
+                         float4 *pos_out, float4 *vel_out, uint32_t *id_out, int *start, cudaStream_t s);
 void launch_scatter_by_id(const uint32_t *id, int64_t n, const float4 *src, float4 *dst, cudaStream_t s);
 void launch_kick_drift(float4 *pos, float4 *vel, const float4 *acc, int64_t n, float dt, BBoxAccum *next_bbox,
                        cudaStream_t s);

@@ -1064,7 +1064,6 @@ void launch_variant(const LaunchArgs &a) {
     blocks = std::min<int64_t>(blocks, a.ws->warps / kWarps);
     blocks = std::min<int64_t>(blocks, (a.ngroups + kWarps - 1) / kWarps);
     if (blocks < 1) blocks = 1;
-    cudaMemsetAsync(a.ws->group_counter, 0, sizeof(unsigned), a.s);
     bh_kernel<ORDER, EPS0, THREADS, PART><<<(unsigned) blocks, THREADS, block_smem_bytes<ORDER, THREADS, PART>(), a.s>>>(
         *a.nodes, a.num_nodes, a.bodies, a.n_bodies, a.targets, a.nt, a.G, a.eps, a.acc, a.counts, a.ws->stack,
         a.ws->group_counter, a.err, a.gtab, (int) a.ngroups, a.inst_root, a.inst_counts);
