@@ -40,6 +40,7 @@
 #include <algorithm>
 #include <cfloat>
 #include <climits>
+#include <cmath>
 
 #include "nb_internal.cuh"
 #include "stensor.cuh"
@@ -378,8 +379,8 @@ constexpr int kItemRoots = 0, kItemBodies = 1;
 // Appends a near-field item for passive leaf `leaf` (bodies [first, first + size)): the payload is
 // a[0..na) then b[0..nb) (activeTree roots), or for close bodies the runs of consecutive indices as
 // (first index, length) pairs. The owning block is the only writer of the leaf's list head, so the
-// list order is the block's task order. The first item of a leaf also registers its 32-target
-// units for the near kernel. Called by every thread of the block.
+// list order is the block's task order. The first item of a leaf also registers its units of
+// at most pool.unit targets for the near kernel. Called by every thread of the block.
 __device__ void append_item(const NearPool &pool, int leaf, int first, int size, int kind, const int *a, int na,
                             const int *b, int nb, uint32_t *err, int *s_slot) {
     const int count = na + nb;
@@ -392,11 +393,11 @@ __device__ void append_item(const NearPool &pool, int leaf, int first, int size,
                   leaf < pool.head_cap;
         const int old = ok ? pool.head[leaf] : -1;
         if (ok && old < 0) {
-            const int nunits = (size + 31) / 32;
+            const int nunits = (size + pool.unit - 1) / pool.unit;
             const unsigned long long u = atomicAdd(&pool.counters[2], (unsigned long long) nunits);
             ok = u + nunits <= (unsigned long long) pool.unit_cap;
             if (ok)
-                for (int j = 0; j < nunits; ++j) pool.units[u + j] = make_int2(leaf, first + 32 * j);
+                for (int j = 0; j < nunits; ++j) pool.units[u + j] = make_int2(leaf, first + pool.unit * j);
         }
         if (ok) {
             pool.items[it] = make_int4(old, kind, (int) off, count);
@@ -1466,7 +1467,7 @@ __global__ void __launch_bounds__(kNearThreads, 8) near_kernel(DualNodes nodes, 
             continue;
         }
         const int2 lr = __ldg(nodes.link + leaf);
-        const int tend = min(lr.y, unit.y + 32);
+        const int tend = min(lr.y, unit.y + pool.unit);
         if (lr.y < 0 || !x.range_ok(unit.y, tend) || tend == unit.y) {
             if (lane == 0) atomicOr(err, (uint32_t) kErrTraverseLimit);
             continue;
@@ -1567,6 +1568,8 @@ __global__ void __launch_bounds__(kNearThreads, 8) near_kernel(DualNodes nodes, 
 
 }  // namespace
 
+constexpr int64_t kSmallDual = 131072;
+
 // Near-field grid: the resident blocks, never more than the walk stacks allocated (one per warp).
 unsigned near_grid(const DualWorkspace &ws) {
     const int64_t by_stacks = ws.near.walk_warps / kNearWarps;
@@ -1586,7 +1589,14 @@ void launch_dual_traverse(const DualNodes &nodes, const int *num_nodes, const fl
     load_balanced_break_kernel<<<1, 512, 0, s>>>(nodes, num_nodes, ws.roots, ws.num_roots, err);
     // passive nodes of at most `frontier` bodies below a larger parent are handed to the second
     // kernel, which balances them over the whole GPU
-    const int frontier = (int) std::max<int64_t>(64, n / 4096);
+    // Measured (whole traversal, theta 0.4 and 0.5, frontier 64 / 128 / 256 / 512 / 1024): 60,001 bodies
+    // 2.94-3.23 / 2.79-3.41 / 3.5-4.4 ms; 250,000: 17.6-19.7 / 15.6-16.8 / 15.2-16.3 / 18.8-19.9 ms; 10^6 at 0.5:
+    // 58.7 (256) / 56.2 / 62.1 ms; 2^22 at 0.4: 365 (256) / 346 / 341 ms.
+    const int frontier = n < kSmallDual ? 64 : (int) (0.5 * std::sqrt((double) n));
+    // Few units leave warps idle and the largest one sets the near field's time: half-size units (two
+    // replicas of each target) below kSmallDual bodies. 60,001 bodies: 3.24 -> 2.82 ms and 3.00 -> 2.56 ms;
+    // 250,000: 17.6 -> 18.1 ms.
+    ws.near.unit = n < kSmallDual ? 16 : 32;
     dual_kernel<false><<<kDualRoots, kThreads, 0, s>>>(nodes, num_nodes, bodies, (int) n, G, eps, theta, acc,
                                                        counts, ws.roots, ws.num_roots, ws.arena, (int) ws.arena_words,
                                                        ws.tasks, ws.near, ws.spill, frontier, lo, hi, err);

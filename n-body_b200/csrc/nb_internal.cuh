@@ -261,7 +261,8 @@ struct NearPool {
     int *head = nullptr;                  // per node: newest item of the passive leaf, -1 if none
     int4 *items = nullptr;                // (next item, kind, payload offset, payload count)
     int *words = nullptr;                 // payload: node or body indices
-    int2 *units = nullptr;                // (passive leaf, first target) per 32-target unit
+    int2 *units = nullptr;                // (passive leaf, first target) per unit of at most `unit` targets
+    int unit = 32;                        // 16 or 32
     unsigned long long *counters = nullptr;  // items, words, units, unit cursor
     int64_t head_cap = 0, item_cap = 0, word_cap = 0, unit_cap = 0;
     int2 *walk_stack = nullptr;           // per warp of the near-field grid: kNearWalkStack (node, mask)
