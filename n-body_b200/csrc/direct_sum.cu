@@ -3,8 +3,8 @@
 //
 // A block of eight warps stages 256 source bodies at a time in shared memory (coalesced float4 loads,
 // double buffered, one barrier per tile) and sweeps the tile with broadcast reads. Its targets:
-//   Z = 8: 32 targets, one per lane, every warp taking an eighth of each tile;
-//   Z = 1: 256 targets, one per thread, for target counts that fill the GPU that way already.
+//   Z = 8: 32 targets (FP32: 64 where there are enough), every warp taking an eighth of each tile;
+//   Z = 1: 256 targets (FP32: 512), for target counts that fill the GPU that way already.
 // Up to eight blocks of a cluster share the sources of the same targets. Partial sums meet in shared
 // memory, warps first, then the cluster's blocks (distributed shared memory), in a fixed order.
 // One thread per target over all sources, 256 targets per block, left 30,011 targets on 118 of 148
@@ -76,9 +76,12 @@ __device__ __forceinline__ bool reduce_target(T (*part)[3], T &ax, T &ay, T &az)
 }
 
 // Bound by the FP32 pipe: 12 lane operations per pair (six paired instructions for two) against a
-// quarter of a lane's reciprocal roots per clock (300 us for 30,011 bodies). 30,011 bodies: 692 us before,
-// 456 us now.
-template<bool EPS0, int Z>
+// quarter of a lane's reciprocal roots per clock (300 us for 30,011 bodies). A broadcast 16-byte read
+// still delivers 512 bytes to the warp's registers, four cycles of the SM's shared-memory pipe: with
+// one target per lane the two reads of a source pair outweigh its arithmetic, so a lane takes T = 2 targets
+// where there are enough of them.
+// 30,011 bodies: 692 us before, 456 us with T = 1, 426 us now.
+template<bool EPS0, int Z, int T>
 __global__ void __launch_bounds__(kThreads) direct_f32_kernel(const float4 *__restrict__ bodies, int64_t n,
                                                               const float4 *__restrict__ targets, int64_t nt,
                                                               float G, float eps, float4 *__restrict__ acc) {
@@ -88,11 +91,18 @@ __global__ void __launch_bounds__(kThreads) direct_f32_kernel(const float4 *__re
     constexpr int kTargets = kThreads / Z;
     cg::cluster_group cluster = cg::this_cluster();
     const int t = threadIdx.x, z = t / kTargets;
-    const int64_t i = (int64_t) (blockIdx.x / cluster.num_blocks()) * kTargets + t % kTargets;
-    const float4 p = i < nt ? targets[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-    const float2 npx = make_float2(-p.x, -p.x), npy = make_float2(-p.y, -p.y), npz = make_float2(-p.z, -p.z);
+    const int64_t i0 = (int64_t) (blockIdx.x / cluster.num_blocks()) * (kTargets * T) + t % kTargets;
+    float2 npx[T], npy[T], npz[T], ax[T], ay[T], az[T];
+#pragma unroll
+    for (int q = 0; q < T; ++q) {
+        const int64_t i = i0 + q * kTargets;
+        const float4 p = i < nt ? targets[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+        npx[q] = make_float2(-p.x, -p.x);
+        npy[q] = make_float2(-p.y, -p.y);
+        npz[q] = make_float2(-p.z, -p.z);
+        ax[q] = ay[q] = az[q] = make_float2(0.f, 0.f);
+    }
     const float2 eps2 = make_float2(eps, eps);
-    float2 ax = make_float2(0.f, 0.f), ay = ax, az = ax;
     int64_t begin, end;
     source_range(n, cluster.block_rank(), cluster.num_blocks(), begin, end);
     float4 next = load_source(bodies, begin + t, end);
@@ -107,17 +117,25 @@ __global__ void __launch_bounds__(kThreads) direct_f32_kernel(const float4 *__re
         next = load_source(bodies, base + kTile + t, end);
         const int pairs = (int) ((end - base < kTile ? end - base : kTile) + 1) >> 1;
         const float4 *src = tile[buf];
+        auto terms = [&](int k) {
+            const float4 u = src[2 * k], v = src[2 * k + 1];
+#pragma unroll
+            for (int q = 0; q < T; ++q) pair2_term<EPS0>(npx[q], npy[q], npz[q], eps2, u, v, ax[q], ay[q], az[q]);
+        };
         if (pairs == kTile / 2) {
-#pragma unroll 8
-            for (int k = z; k < kTile / 2; k += Z)
-                pair2_term<EPS0>(npx, npy, npz, eps2, src[2 * k], src[2 * k + 1], ax, ay, az);
+#pragma unroll 4
+            for (int k = z; k < kTile / 2; k += Z) terms(k);
         } else {
-            for (int k = z; k < pairs; k += Z)
-                pair2_term<EPS0>(npx, npy, npz, eps2, src[2 * k], src[2 * k + 1], ax, ay, az);
+            for (int k = z; k < pairs; k += Z) terms(k);
         }
     }
-    float sx = ax.x + ax.y, sy = ay.x + ay.y, sz = az.x + az.y;
-    if (reduce_target<Z>(part, sx, sy, sz) && i < nt) acc[i] = make_float4(G * sx, G * sy, G * sz, 0.f);
+#pragma unroll
+    for (int q = 0; q < T; ++q) {
+        const int64_t i = i0 + q * kTargets;
+        float sx = ax[q].x + ax[q].y, sy = ay[q].x + ay[q].y, sz = az[q].x + az[q].y;
+        if (q > 0) __syncthreads();  // the target before has been added up
+        if (reduce_target<Z>(part, sx, sy, sz) && i < nt) acc[i] = make_float4(G * sx, G * sy, G * sz, 0.f);
+    }
 }
 
 // 1 / sqrt(x) of a normal x > 0 in FP64: the hardware's seed (relative error below 2^-19) and one step of
@@ -310,6 +328,8 @@ void launch_clusters(void (*kernel)(Params...), int64_t target_blocks, int clust
 // From this many targets on, 256 per block fill the GPU for several waves, and sources are read from
 // L2 once per 256 targets instead of once per 32.
 constexpr int64_t kWideTargets = 300000;
+// From this many targets on, two per lane leave enough blocks.
+constexpr int64_t kPairTargets = 8192;
 
 }  // namespace
 
@@ -326,15 +346,16 @@ void launch_energy_f64(const float4 *bodies, const float4 *vel, int64_t n, doubl
 void launch_direct_f32(const float4 *bodies, int64_t n, const float4 *targets, int64_t nt, int64_t shape_targets,
                        float G, float eps, float4 *acc, cudaStream_t s) {
     if (nt <= 0) return;
-    if (shape_targets >= kWideTargets) {
-        const int64_t blocks = (nt + kThreads - 1) / kThreads;
-        auto kernel = eps == 0.f ? direct_f32_kernel<true, 1> : direct_f32_kernel<false, 1>;
-        launch_clusters(kernel, blocks, 1, s, bodies, n, targets, nt, G, eps, acc);
-    } else {
-        const int64_t blocks = (nt + 31) / 32;
-        auto kernel = eps == 0.f ? direct_f32_kernel<true, 8> : direct_f32_kernel<false, 8>;
-        launch_clusters(kernel, blocks, cluster_for((shape_targets + 31) / 32, n), s, bodies, n, targets, nt, G, eps, acc);
-    }
+    auto launch = [&](auto narrow, auto soft, int per_block, int cluster) {
+        launch_clusters(eps == 0.f ? narrow : soft, (nt + per_block - 1) / per_block, cluster, s, bodies, n, targets, nt, G,
+                        eps, acc);
+    };
+    if (shape_targets >= kWideTargets)
+        launch(direct_f32_kernel<true, 1, 2>, direct_f32_kernel<false, 1, 2>, 2 * kThreads, 1);
+    else if (shape_targets >= kPairTargets)
+        launch(direct_f32_kernel<true, 8, 2>, direct_f32_kernel<false, 8, 2>, 64, cluster_for((shape_targets + 63) / 64, n));
+    else
+        launch(direct_f32_kernel<true, 8, 1>, direct_f32_kernel<false, 8, 1>, 32, cluster_for((shape_targets + 31) / 32, n));
 }
 
 void launch_direct_f64(const float4 *bodies, int64_t n, const float4 *targets, int64_t nt, double G, double eps,

@@ -19,7 +19,7 @@ def reference(bodies, targets, eps):
     return terms.sum(1), np.abs(terms).sum(1)
 
 
-@pytest.mark.parametrize("n,nt", [(1, 1), (2, 33), (255, 31), (256, 32), (257, 300), (1025, 1), (4097, 513), (20011, 64)])
+@pytest.mark.parametrize("n,nt", [(1, 1), (2, 33), (255, 31), (256, 32), (257, 300), (1025, 1), (4097, 513), (20011, 64), (700, 8191), (700, 8192), (700, 8257)])
 @pytest.mark.parametrize("eps", [0.0, 1e-4])
 def test_direct_sums(nb, n, nt, eps):
     import torch
