@@ -48,6 +48,21 @@ __global__ void __launch_bounds__(kThreads) scatter_by_id_kernel(const uint32_t 
     if (d < (uint64_t) n) dst[d] = src[k];
 }
 
+__global__ void __launch_bounds__(kThreads) collect_kernel(const uint32_t *__restrict__ id, int64_t n, int64_t first,
+                                                           const float4 *__restrict__ pos, const float4 *__restrict__ vel,
+                                                           float4 *__restrict__ pos_out, float4 *__restrict__ vel_out,
+                                                           uint32_t *__restrict__ err) {
+    const int64_t k = (int64_t) blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= n) return;
+    const int64_t d = (int64_t) id[k] - first;
+    if (d < 0 || d >= n) {
+        atomicOr(err, (uint32_t) kErrServedIds);
+        return;
+    }
+    pos_out[d] = pos[k];
+    vel_out[d] = vel[k];
+}
+
 __global__ void __launch_bounds__(kThreads) iota_kernel(uint32_t *__restrict__ id, int64_t n, uint32_t first) {
     const int64_t k = (int64_t) blockIdx.x * blockDim.x + threadIdx.x;
     if (k < n) id[k] = first + (uint32_t) k;
@@ -116,6 +131,12 @@ void launch_gather_state(const uint32_t *perm, int64_t n, const float4 *pos, con
 void launch_scatter_by_id(const uint32_t *id, int64_t n, const float4 *src, float4 *dst, cudaStream_t s) {
     if (n <= 0) return;
     scatter_by_id_kernel<<<blocks_for(n), kThreads, 0, s>>>(id, n, src, dst);
+}
+
+void launch_collect(const uint32_t *id, int64_t n, int64_t first, const float4 *pos, const float4 *vel, float4 *pos_out,
+                    float4 *vel_out, uint32_t *err, cudaStream_t s) {
+    if (n <= 0) return;
+    collect_kernel<<<blocks_for(n), kThreads, 0, s>>>(id, n, first, pos, vel, pos_out, vel_out, err);
 }
 
 void launch_iota(uint32_t *id, int64_t n, cudaStream_t s, uint32_t first) {

@@ -146,6 +146,7 @@ enum DeviceError : uint32_t {
     kErrStackOverflow = 1u << 3,     // traversal stack full (a push was dropped)
     kErrTraverseLimit = 1u << 4,     // traversal met an invalid link or exceeded its round limit
     kErrDualArena = 1u << 5,         // dual-tree list or task storage exhausted
+    kErrServedIds = 1u << 7,         // a served request's body id lies outside its range
     kErrNearPool = 1u << 6,          // dual-tree near-field pool too small (the host grows it and retries)
 };
 
@@ -351,6 +352,9 @@ void launch_scatter_by_id(const uint32_t *id, int64_t n, const float4 *src, floa
 void launch_kick_drift(float4 *pos, float4 *vel, const float4 *acc, int64_t n, float dt, BBoxAccum *next_bbox,
                        cudaStream_t s);
 void launch_iota(uint32_t *id, int64_t n, cudaStream_t s, uint32_t first = 0);
+// Bodies of one instance (ids first .. first + n - 1) into their id order; an id outside sets kErrServedIds.
+void launch_collect(const uint32_t *id, int64_t n, int64_t first, const float4 *pos, const float4 *vel, float4 *pos_out,
+                    float4 *vel_out, uint32_t *err, cudaStream_t s);
 void launch_add_offset(uint32_t *id, int64_t n, int64_t delta, cudaStream_t s);
 
 // batch.cu
