@@ -75,7 +75,8 @@ __device__ __forceinline__ void store_volatile(uint32_t *p, uint32_t v) { *(vola
 // store their keys straight into the shared memory of the block that holds their new position
 // (distributed shared memory): two cluster barriers per pass instead of a kernel with its look-back.
 // Latency bound. 1,023 keys: 49 us in eight one-sweep launches before, 20 us now; 10,000 keys: 68 and
-// 43 us. One block of 1,024 threads instead of the cluster: 28 and 143 us.
+// 37 us (43 us when keys went straight from their lanes to scattered places of the other blocks). One
+// block of 1,024 threads instead of the cluster: 28 and 143 us.
 constexpr int kCluster = 8;
 constexpr int kClusterThreads = 512;
 constexpr int kClusterWarps = kClusterThreads / 32;
@@ -84,8 +85,11 @@ template<int K>
 struct ClusterSmem {
     uint64_t keys[kClusterThreads * K];
     uint32_t vals[kClusterThreads * K];
-    uint32_t hist[kClusterWarps][256];  // per warp: digit counts, then its keys' new positions
+    uint64_t stage_keys[kClusterThreads * K];  // the block's keys in digit order
+    uint32_t stage_vals[kClusterThreads * K];
+    uint32_t hist[kClusterWarps][256];  // per warp: digit counts, then its keys' places in the block
     uint32_t count[256];                // the block's digit counts, read by the other blocks
+    uint32_t shift[256];                // per digit: place in the cluster minus place in the block
     uint32_t total[8];
 };
 
@@ -136,15 +140,17 @@ __global__ void __launch_bounds__(kClusterThreads) __cluster_dims__(kCluster, 1,
             S.count[tid] = sum;
         }
         cluster.sync();
-        uint32_t total = 0, before = 0, incl = 0;
+        // one scan over the digits for both: the cluster's counts (upper half) and the block's
+        uint32_t packed = 0, before = 0, incl = 0;
         if (tid < 256) {
 #pragma unroll
             for (int b = 0; b < kCluster; ++b) {
                 const uint32_t x = *cluster.map_shared_rank(&S.count[tid], b);
-                total += x;
+                packed += x << 16;
                 if (b < rank) before += x;
             }
-            incl = total;
+            packed += sum;
+            incl = packed;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
                 const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
@@ -154,22 +160,35 @@ __global__ void __launch_bounds__(kClusterThreads) __cluster_dims__(kCluster, 1,
         }
         __syncthreads();
         if (tid < 256) {
-            uint32_t run = incl - total + before;
+            uint32_t run = incl - packed;
 #pragma unroll
             for (int w = 0; w < 8; ++w) run += w < warp ? S.total[w] : 0u;
+            uint32_t place = run & 0xffffu;
+            S.shift[tid] = (run >> 16) + before - place;
 #pragma unroll
             for (int w = 0; w < kClusterWarps; ++w) {
-                S.hist[w][tid] = run;
-                run += c[w];
+                S.hist[w][tid] = place;
+                place += c[w];
             }
+        }
+        __syncthreads();
+        // in digit order within the block first, so that neighbouring threads store to neighbouring
+        // places of the other blocks: single stores to scattered ones took most of a pass
+#pragma unroll
+        for (int it = 0; it < K; ++it) {
+            const uint32_t at = S.hist[warp][(uint32_t) (k[it] >> shift) & 255u] + r[it];
+            S.stage_keys[at] = k[it];
+            S.stage_vals[at] = v[it];
         }
         __syncthreads();
 #pragma unroll
         for (int it = 0; it < K; ++it) {
-            const uint32_t pos = S.hist[warp][(uint32_t) (k[it] >> shift) & 255u] + r[it];
+            const int i = it * kClusterThreads + tid;
+            const uint64_t key = S.stage_keys[i];
+            const uint32_t pos = i + S.shift[(uint32_t) (key >> shift) & 255u];
             const unsigned to = pos / kBlockKeys, at = pos % kBlockKeys;
-            *cluster.map_shared_rank(&S.keys[at], to) = k[it];
-            *cluster.map_shared_rank(&S.vals[at], to) = v[it];
+            *cluster.map_shared_rank(&S.keys[at], to) = key;
+            *cluster.map_shared_rank(&S.vals[at], to) = S.stage_vals[i];
         }
         cluster.sync();
 #pragma unroll
