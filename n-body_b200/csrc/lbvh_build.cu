@@ -17,7 +17,7 @@
 //                     and the number of final nodes starting at each body position
 //   scan kernels      exclusive prefix over body positions of those counts: the preorder index of
 //                     the final leaf starting at each position
-//   summarize_kernel  one block per kClimbNodes Karras nodes, one thread per final internal node with
+//   summarize_kernel  one block per 1024 or 4096 Karras nodes, one thread per final internal node with
 //                     leaf children: sequential leaf summaries over the leaf's bodies, then a climb in
 //                     which the second child to arrive summarises the parent (CenterOfMassSummary.h:30-55,
 //                     BoundingBoxSummary.h:30-68, MultipoleMassSummary.h:37-97; the leaf moment
@@ -639,33 +639,36 @@ __device__ __forceinline__ Summ<ORDER> combine(const TreeWorkspace &tw, const Su
                                                                               : internal_summary<ORDER>(l, r);
 }
 
-// One block per kClimbNodes Karras nodes. All descendants of a node that covers bodies [first, last] have
+// One block per NODES Karras nodes. All descendants of a node that covers bodies [first, last] have
 // Karras indices in [first, last], so a node whose range lies in the block's index range is climbed
 // to by this block's threads alone: its arrivals are counted in shared memory and need block-scope
 // ordering only, a few hundred cycles instead of the device-scope arrival's round trips to L2.
-constexpr int kClimbNodes = 1024;
+// 1024 nodes hold enough leaf parents for 128 threads at leaves of up to some 16 bodies; larger leaves
+// take 4096 (2^22 bodies at leaf 64, octupole: 0.77 ms with 1024).
 constexpr int kClimbThreads = 128;
-static_assert(kClimbNodes == 8 * kClimbThreads, "eight node flags per thread");
+constexpr int kClimbSmall = 1024, kClimbLarge = 4096;
 
+template<int NODES>
 struct ClimbSmem {
-    int visit[kClimbNodes];
-    uint16_t list[2][kClimbNodes];  // the block's final internal nodes: those with leaf children, all of them
+    int visit[NODES];
+    uint16_t list[2][NODES];  // the block's final internal nodes: those with leaf children, all of them
     int count[2];
 };
 
+template<int NODES>
 __device__ __forceinline__ bool in_block(int4 tp) {
-    const int lo = blockIdx.x * kClimbNodes;
-    return tp.z >= lo && tp.w < lo + kClimbNodes;
+    const int lo = blockIdx.x * NODES;
+    return tp.z >= lo && tp.w < lo + NODES;
 }
 
 // Final internal node i's final-leaf children: leaf summaries, then the climb. A node whose children
 // are both final leaves is finished at once, without an arrival. The topology of the next node up is
 // loaded while the current level computes. Records of nodes beyond the block's own are written on
 // the way, after the arrival at the parent.
-template<int ORDER, class Records>
+template<int ORDER, int NODES, class Records>
 __device__ void summarize_from(const float4 *__restrict__ bodies, int n, const TreeWorkspace &tw, uint32_t *err,
-                               const Records &rec, ClimbSmem &S, int i) {
-    const int lo = blockIdx.x * kClimbNodes;
+                               const Records &rec, ClimbSmem<NODES> &S, int i) {
+    const int lo = blockIdx.x * NODES;
     int4 tp = tw.topo[i];  // (left child, right child, first body, last body) of the node p below
     uint8_t fl = tw.flags[i];
     int par = tw.parent[i];  // not written for the root, and read only below a non-root node
@@ -682,7 +685,7 @@ __device__ void summarize_from(const float4 *__restrict__ bodies, int n, const T
         mine = combine<ORDER>(tw, l, r, tp.z, tp.w);
         store_slot<ORDER>(tw, i, mine);
         tw.chain[i] = 0;
-        if (!in_block(tp)) {
+        if (!in_block<NODES>(tp)) {
             pending = true;
             right_pre = preorder_leaf(tw, gamma + 1);
             pre = preorder_internal(tw, tp.z, 0);
@@ -716,7 +719,7 @@ __device__ void summarize_from(const float4 *__restrict__ bodies, int n, const T
             atomicOr(err, (uint32_t) kErrTreeDepth);
             return;
         }
-        const bool own = in_block(tp);
+        const bool own = in_block<NODES>(tp);
         bool second;
         if (own) {
             __threadfence_block();
@@ -773,13 +776,13 @@ __device__ void summarize_from(const float4 *__restrict__ bodies, int n, const T
 }
 
 // Records of the block's final internal node i, if the block finished it, and of its final-leaf children.
-template<int ORDER, class Records>
+template<int ORDER, int NODES, class Records>
 __device__ void write_records(int n, const TreeWorkspace &tw, uint32_t *err, const Records &rec, int i) {
     const int4 tp = tw.topo[i];
     const uint8_t fl = tw.flags[i];
     const int gamma = tp.x >= 0 ? tp.x : ~tp.x;
     const bool lfin = (fl & kLeftLeaf) != 0, rfin = (fl & kRightLeaf) != 0;
-    if (in_block(tp)) {
+    if (in_block<NODES>(tp)) {
         const int right_pre = rfin ? preorder_leaf(tw, gamma + 1) : preorder_internal(tw, gamma + 1, __ldcg(tw.chain + tp.y));
         rec.internal(preorder_internal(tw, tp.z, __ldcg(tw.chain + i)), load_slot<ORDER>(tw, i), tp.z, tp.w, right_pre, err);
     }
@@ -794,12 +797,13 @@ __device__ void write_records(int n, const TreeWorkspace &tw, uint32_t *err, con
 // over the nodes in between. The whole tree is one leaf when n == 1, or when the root is not
 // splittable (n <= maxLeafSize or every code equal): the first block's first thread writes it.
 // Cold-cache times, before (device-scope arrivals at every level, records on the chain, a list of leaf
-// parents made by karras_kernel) and now: 1,023 bodies 66 and 47 us, 60,001 bodies (octupole) 160 and 141 us, 2^20
-// bodies 112 and 145 us with karras_kernel 73 and 46 us; four launches and clears fewer per build.
-template<int ORDER, class Records>
+// parents made by karras_kernel) and now: 1,023 bodies 66 and 47 us, 10,000 (monopole) 46 and 52 us, 2^20 bodies 112
+// and 145 us with karras_kernel 73 and 46 us, 9.3 million bodies in 256 instances 2.65 and 0.77 ms; four launches
+// and clears fewer per build.
+template<int ORDER, int NODES, class Records>
 __global__ void __launch_bounds__(kClimbThreads) summarize_kernel(const float4 *__restrict__ bodies, int n, TreeWorkspace tw,
                                                                   uint32_t *err, Records rec) {
-    __shared__ ClimbSmem S;
+    __shared__ ClimbSmem<NODES> S;
     if (n == 1 || !(tw.flags[0] & kFinal)) {
         if (blockIdx.x == 0 && threadIdx.x == 0) {
             rec.leaf(0, leaf_summary<ORDER>(bodies, 0, n - 1), 0, n - 1, err);
@@ -807,12 +811,13 @@ __global__ void __launch_bounds__(kClimbThreads) summarize_kernel(const float4 *
         }
         return;
     }
-    const int lo = blockIdx.x * kClimbNodes, count = min(kClimbNodes, n - 1 - lo);
+    const int lo = blockIdx.x * NODES, count = min(NODES, n - 1 - lo);
     if (threadIdx.x == 0) S.count[0] = S.count[1] = 0;
     for (int k = threadIdx.x; k < count; k += kClimbThreads) S.visit[k] = 0;
     __syncthreads();
-    {   // eight flags per thread in one load (the flags are padded to a multiple of eight)
-        const int k0 = 8 * threadIdx.x;
+#pragma unroll
+    for (int k0 = 8 * threadIdx.x; k0 < NODES; k0 += 8 * kClimbThreads) {
+        // eight flags in one load (the flags are padded to a multiple of eight)
         const uint64_t eight = k0 < count ? *reinterpret_cast<const uint64_t *>(tw.flags + lo + k0) : 0ull;
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
@@ -823,13 +828,21 @@ __global__ void __launch_bounds__(kClimbThreads) summarize_kernel(const float4 *
     }
     __syncthreads();
     for (int k = threadIdx.x; k < S.count[0]; k += kClimbThreads)
-        summarize_from<ORDER, Records>(bodies, n, tw, err, rec, S, lo + S.list[0][k]);
+        summarize_from<ORDER, NODES, Records>(bodies, n, tw, err, rec, S, lo + S.list[0][k]);
     __syncthreads();
     for (int k = threadIdx.x; k < S.count[1]; k += kClimbThreads)
-        write_records<ORDER, Records>(n, tw, err, rec, lo + S.list[1][k]);
+        write_records<ORDER, NODES, Records>(n, tw, err, rec, lo + S.list[1][k]);
 }
 
-int summarize_blocks(int n) { return std::max(1, (n - 1 + kClimbNodes - 1) / kClimbNodes); }
+template<int ORDER, class Records>
+void launch_summarize(const float4 *bodies, int n, int leaf, const TreeWorkspace &tw, uint32_t *err, cudaStream_t s,
+                      const Records &rec) {
+    auto blocks = [n](int nodes) { return (unsigned) std::max(1, (n - 1 + nodes - 1) / nodes); };
+    if (leaf > 16)
+        summarize_kernel<ORDER, kClimbLarge, Records><<<blocks(kClimbLarge), kClimbThreads, 0, s>>>(bodies, n, tw, err, rec);
+    else
+        summarize_kernel<ORDER, kClimbSmall, Records><<<blocks(kClimbSmall), kClimbThreads, 0, s>>>(bodies, n, tw, err, rec);
+}
 
 // Karras topology, the final nodes per start position (tw.start is zero on entry) and their
 // exclusive prefix (which also gives the node count); the topology kernel also clears the climb's
@@ -867,8 +880,7 @@ void launch_build_dual_tree(const uint64_t *sorted_codes, const float4 *bodies, 
         return;
     }
     if (n > 1) launch_topology(sorted_codes, nullptr, n, leaf, tw, s);
-    summarize_kernel<3, DualRecords>
-        <<<summarize_blocks(n), kClimbThreads, 0, s>>>(bodies, n, tw, err, DualRecords{nodes, theta});
+    launch_summarize<3>(bodies, n, leaf, tw, err, s, DualRecords{nodes, theta});
 }
 
 void launch_build_tree(const uint64_t *sorted_codes, const float4 *bodies, int64_t n64, int leaf, int order,
@@ -882,11 +894,9 @@ void launch_build_tree(const uint64_t *sorted_codes, const float4 *bodies, int64
     const float t = theta * theta;  // the reference compares against theta * theta in float
     if (n > 1) launch_topology(sorted_codes, seg.inst_of, n, leaf, tw, s);
     if (order == 1)
-        summarize_kernel<1, BhRecords<1>>
-            <<<summarize_blocks(n), kClimbThreads, 0, s>>>(bodies, n, tw, err, BhRecords<1>{nodes, t, seg});
+        launch_summarize<1>(bodies, n, leaf, tw, err, s, BhRecords<1>{nodes, t, seg});
     else
-        summarize_kernel<2, BhRecords<2>>
-            <<<summarize_blocks(n), kClimbThreads, 0, s>>>(bodies, n, tw, err, BhRecords<2>{nodes, t, seg});
+        launch_summarize<2>(bodies, n, leaf, tw, err, s, BhRecords<2>{nodes, t, seg});
 }
 
 }  // namespace nbg
