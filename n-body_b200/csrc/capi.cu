@@ -1585,7 +1585,9 @@ int nb_server_tick(nb_server *sv, int32_t *completed_now) {
     }
     int32_t completed = 0;
     bool changed = sv->dirty;
-    // 1. retire requests whose steps are done, drop cancelled ones
+    // 1. retire requests whose steps are done, drop cancelled ones. One that cannot be copied out stays in
+    // the running set (until it is cancelled) and fails the tick, once the others have been retired.
+    int failed = NB_OK;
     std::vector<ServedRequest *> keep;
     for (auto *r: sv->active) {
         if (r->cancel) {
@@ -1594,8 +1596,12 @@ int nb_server_tick(nb_server *sv, int32_t *completed_now) {
             sv->stats.cancelled += 1;
             changed = true;
         } else if (r->done >= r->steps) {
-            int rc = server_collect(sv, r);
-            if (rc != NB_OK) return rc;
+            const int rc = server_collect(sv, r);
+            if (rc != NB_OK) {
+                failed = rc;
+                keep.push_back(r);
+                continue;
+            }
             r->state = 2;
             r->start = -1;
             ++completed;
@@ -1605,6 +1611,14 @@ int nb_server_tick(nb_server *sv, int32_t *completed_now) {
         }
     }
     sv->active.swap(keep);
+    if (failed != NB_OK) {
+        sv->dirty = changed;
+        sv->stats.completed += completed;
+        sv->stats.failed_ticks += 1;
+        sv->stats.running = (int64_t) sv->active.size();
+        if (completed_now) *completed_now = completed;
+        return failed;
+    }
     // 2. admit queued requests in arrival order while they fit the budget
     uint64_t resident = 0;
     for (auto *r: sv->active) resident += (uint64_t) r->n * kResidentBytesPerBody;

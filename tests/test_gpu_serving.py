@@ -142,3 +142,40 @@ def test_allocation_failure_keeps_server_consistent(nb, point):
     refs = [alone(nb, *small[0], 0.5, 5), alone(nb, *small[1], 0.6, 5), alone(nb, *big, 0.5, 3)]
     for (p, v), (pr, vr) in zip(results, refs):
         assert np.array_equal(p, pr) and np.array_equal(v, vr)
+
+
+def mix_up(nb, sv, n, seed):
+    """Replaces the bodies of the server's three requests of n bodies through its context, and sorts them as one
+    set: the first request's bodies come first and keep their ids, the other two's interleave."""
+    rng = np.random.default_rng(seed)
+    pm = np.full((3 * n, 4), 1.0 / n, np.float32)
+    pm[:, :3] = rng.uniform(0.75, 1.0, (3 * n, 3))
+    pm[:n, :3] -= 0.75
+    lib, ctx = nb.lib(), sv.context()
+    assert lib.nb_set_bodies(ctx, 3 * n, pm.ctypes.data, None) == nb.NB_OK
+    assert lib.nb_update_accelerations(ctx, None) == nb.NB_OK
+    return pm
+
+
+def test_a_request_that_cannot_be_copied_out_fails_alone(nb):
+    """Two of three finished requests have ids of other requests: the tick reports it, the third is retired, a
+    cancelled one is dropped once, and the requests left are neither copied out again nor lost."""
+    n = 100
+    with nb.Server(rule=nb.Gravity(1.0, EPS), time_step=DT) as sv:
+        ids = [sv.submit(*nb.scenarios.plummer(n, seed=90 + k), theta=0.5, steps=1) for k in range(3)]
+        sv.tick()
+        pm = mix_up(nb, sv, n, seed=1)
+        with pytest.raises(nb.NBodyError):
+            sv.tick()
+        assert [sv.status(r)[0] for r in ids] == [nb.Server.DONE, nb.Server.RUNNING, nb.Server.RUNNING]
+        sv.cancel(ids[1])
+        for _ in range(2):  # the last one still cannot be copied out
+            with pytest.raises(nb.NBodyError):
+                sv.tick()
+        with pytest.raises(nb.NBodyError):
+            sv.status(ids[1])
+        sv.cancel(ids[2])
+        sv.tick()
+        st = sv.stats()
+        assert (st["completed"], st["cancelled"], st["failed_ticks"], st["running"]) == (1, 2, 3, 0)
+        assert np.array_equal(sv.take_result(ids[0], n)[0], pm[:n])
