@@ -571,7 +571,6 @@ int device_status(nb_ctx *ctx) {
     if (e & kErrTraverseLimit) return fail(ctx, NB_ERR_DEVICE_CHECK, "traversal met an invalid tree link");
     if (e & kErrDualArena) return fail(ctx, NB_ERR_DEVICE_CHECK, "dual-tree list or task storage exhausted");
     if (e & kErrNearPool) return fail(ctx, NB_ERR_DEVICE_CHECK, "dual-tree near-field pool exhausted");
-    if (e & kErrServedIds) return fail(ctx, NB_ERR_DEVICE_CHECK, "corrupt body ids in a served request");
     return NB_OK;
 }
 
@@ -1501,6 +1500,13 @@ static int server_collect(nb_server *sv, ServedRequest *r) {
         return NB_ERR_CUDA;
     }
     if (e & kErrServedIds) {
+        // reported with this request: the context and the other requests' copies are not affected
+        e &= ~(uint32_t) kErrServedIds;
+        if (cudaMemcpyAsync(ctx->err, &e, sizeof(e), cudaMemcpyHostToDevice, s) != cudaSuccess ||
+            cudaStreamSynchronize(s) != cudaSuccess) {
+            sv->error = "copy-out failed";
+            return NB_ERR_CUDA;
+        }
         sv->error = "corrupt body ids in a served request";
         return NB_ERR_DEVICE_CHECK;
     }

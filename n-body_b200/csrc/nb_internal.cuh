@@ -146,8 +146,8 @@ enum DeviceError : uint32_t {
     kErrStackOverflow = 1u << 3,     // traversal stack full (a push was dropped)
     kErrTraverseLimit = 1u << 4,     // traversal met an invalid link or exceeded its round limit
     kErrDualArena = 1u << 5,         // dual-tree list or task storage exhausted
-    kErrServedIds = 1u << 7,         // a served request's body id lies outside its range
     kErrNearPool = 1u << 6,          // dual-tree near-field pool too small (the host grows it and retries)
+    kErrServedIds = 1u << 7,         // a served request's body id lies outside its range (cleared when reported)
 };
 
 // ---- launchers (stream-ordered; defined in the .cu files) ----

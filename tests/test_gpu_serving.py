@@ -179,3 +179,25 @@ def test_a_request_that_cannot_be_copied_out_fails_alone(nb):
         st = sv.stats()
         assert (st["completed"], st["cancelled"], st["failed_ticks"], st["running"]) == (1, 2, 3, 0)
         assert np.array_equal(sv.take_result(ids[0], n)[0], pm[:n])
+
+
+def test_a_reported_copy_out_failure_is_over(nb):
+    """Once the requests with ids of other requests are cancelled, the context's status is clean and a new
+    request runs and ends as it does alone."""
+    n = 100
+    with nb.Server(rule=nb.Gravity(1.0, EPS), time_step=DT) as sv:
+        ids = [sv.submit(*nb.scenarios.plummer(n, seed=90 + k), theta=0.5, steps=1) for k in range(3)]
+        sv.tick()
+        mix_up(nb, sv, n, seed=2)
+        with pytest.raises(nb.NBodyError):
+            sv.tick()
+        assert nb.lib().nb_synchronize(sv.context()) == nb.NB_OK
+        for r in ids[1:]:
+            sv.cancel(r)
+        pm, vel = nb.scenarios.plummer(3 * n, seed=93)
+        r = sv.submit(pm, vel, theta=0.5, steps=2)
+        for _ in range(3):
+            sv.tick()
+        out = sv.take_result(r, 3 * n)
+    ref = alone(nb, pm, vel, 0.5, 2)
+    assert np.array_equal(out[0], ref[0]) and np.array_equal(out[1], ref[1])
