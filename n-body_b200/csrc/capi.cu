@@ -566,6 +566,7 @@ int device_status(nb_ctx *ctx) {
     if (e & kErrLookbackTimeout)
         return fail(ctx, NB_ERR_DEVICE_TIMEOUT, "radix sort look-back wait exceeded its limit");
     if (e & kErrNodeOverflow) return fail(ctx, NB_ERR_DEVICE_CHECK, "tree node buffer overflow");
+    if (e & kErrTeamTimeout) return fail(ctx, NB_ERR_DEVICE_TIMEOUT, "traversal team wait exceeded its limit");
     if (e & kErrTreeDepth) return fail(ctx, NB_ERR_DEVICE_CHECK, "tree walk exceeded the maximum depth");
     if (e & kErrStackOverflow) return fail(ctx, NB_ERR_DEVICE_CHECK, "traversal stack overflow");
     if (e & kErrTraverseLimit) return fail(ctx, NB_ERR_DEVICE_CHECK, "traversal met an invalid tree link");
@@ -1215,9 +1216,11 @@ int nb_selftest_bounded_wait(int32_t device, int32_t wait_ms) {
         return NB_ERR_CUDA;
     }
     if (cudaSetDevice(device) != cudaSuccess) return NB_ERR_CUDA;
-    uint32_t e = 0;
-    if (lookback_timeout_selftest((unsigned long long) wait_ms * 1000000ull, &e) != cudaSuccess) return NB_ERR_CUDA;
-    return (e & kErrLookbackTimeout) ? NB_ERR_DEVICE_TIMEOUT : NB_OK;
+    uint32_t sort = 0, team = 0;
+    const unsigned long long limit_ns = (unsigned long long) wait_ms * 1000000ull;
+    if (lookback_timeout_selftest(limit_ns, &sort) != cudaSuccess) return NB_ERR_CUDA;
+    if (team_timeout_selftest(limit_ns, &team) != cudaSuccess) return NB_ERR_CUDA;
+    return sort == kErrLookbackTimeout && team == kErrTeamTimeout ? NB_ERR_DEVICE_TIMEOUT : NB_OK;
 }
 
 int nb_set_traversal_shape(nb_ctx *ctx, int32_t block_threads, int32_t slab_entries) {

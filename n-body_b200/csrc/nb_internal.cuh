@@ -29,6 +29,13 @@ __device__ __forceinline__ float rsqrt_hw(float x) {
     return y;
 }
 
+// Nanoseconds, for the limits of device-side waits.
+__device__ __forceinline__ unsigned long long global_timer_ns() {
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
+}
+
 // Gravity::particleParticle (Gravity.h:199-209) without G for one target and two sources at once,
 // in paired FP32 arithmetic (sm_100 FADD2 / FFMA2 / FMUL2: one instruction for both halves):
 // u = (x_a, x_b, y_a, y_b), v = (z_a, z_b, m_a, m_b), np = -p in both halves. Per half:
@@ -148,6 +155,7 @@ enum DeviceError : uint32_t {
     kErrDualArena = 1u << 5,         // dual-tree list or task storage exhausted
     kErrNearPool = 1u << 6,          // dual-tree near-field pool too small (the host grows it and retries)
     kErrServedIds = 1u << 7,         // a served request's body id lies outside its range (cleared when reported)
+    kErrTeamTimeout = 1u << 8,       // a traversal team's wait ran out
 };
 
 // ---- launchers (stream-ordered; defined in the .cu files) ----
@@ -326,6 +334,10 @@ int64_t traverse_resident_warps(int device);
 // consecutive groups of 32 that start at node 0. inst_counts (optional, with groups): per instance,
 // (particle-particle, node-particle) interaction counts are added at [2 * instance + {0, 1}]. leaf:
 // the tree's largest leaf (it moves the line between the traversal's two forms, nothing else).
+// Self-test of the team form's bounded waits: one group whose walk hands no leaf list over for several
+// times wait_limit_ns (100 ms at most), so that the warps waiting for one give up. The error word it
+// leaves is returned (kErrTeamTimeout expected).
+cudaError_t team_timeout_selftest(unsigned long long wait_limit_ns, uint32_t *err_word);
 void launch_bh_traverse(int order, const NodeArrays &nodes, const int *num_nodes, const float4 *bodies, int64_t n_bodies,
                         const float4 *targets, int64_t n_targets, int leaf, float G, float eps, float4 *acc,
                         unsigned long long *counts, TraverseWorkspace &ws, uint32_t *err, cudaStream_t s,

@@ -41,12 +41,6 @@ constexpr uint32_t kValueMask = (1u << 30) - 1;
 constexpr int kLook = 4;  // tiles looked back over at a time
 constexpr unsigned long long kWaitLimitNs = 2000000000ull;
 
-__device__ __forceinline__ unsigned long long global_timer_ns() {
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-
 __device__ __forceinline__ uint32_t lanemask_lt() {
     uint32_t m;
     asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));

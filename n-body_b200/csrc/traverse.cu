@@ -40,6 +40,8 @@
 #include <algorithm>
 #include <cfloat>
 #include <climits>
+#include <memory>
+#include <new>
 
 #include "nb_internal.cuh"
 
@@ -483,6 +485,9 @@ constexpr int kLeafRing = 8;
 constexpr int kTeamWarps = 2 + kLeafSets;    // walker, node evaluator, one warp per leaf set
 constexpr int kTeamThreads = 32 * kTeamWarps;
 constexpr int kTeamBlocks = 4;               // resident per SM, by shared memory
+// Limit of one wait. The longest that a sound pass can need is one warp's evaluation of a list that holds every
+// body (coincident bodies make one leaf): about 4 s at 3e8 bodies.
+constexpr unsigned long long kTeamWaitNs = 10000000000ull;
 
 template<int PAY, int PART>
 struct TeamSmem {
@@ -509,22 +514,27 @@ __device__ __forceinline__ void mbar_init(unsigned long long *bar, unsigned coun
 __device__ __forceinline__ void mbar_arrive(unsigned long long *bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"((uint32_t) __cvta_generic_to_shared(bar)) : "memory");
 }
+// One try suspends the warp for at most kTryNs (a hint: without it the time is the system's choice).
+constexpr unsigned kTryNs = 20000;
 __device__ __forceinline__ bool mbar_try_wait(unsigned long long *bar, unsigned parity) {
     unsigned ok;
-    asm volatile("{\n .reg .pred q;\n mbarrier.try_wait.parity.shared::cta.b64 q, [%1], %2;\n selp.u32 %0, 1, 0, q;\n}"
-                 : "=r"(ok) : "r"((uint32_t) __cvta_generic_to_shared(bar)), "r"(parity) : "memory");
+    asm volatile("{\n .reg .pred q;\n mbarrier.try_wait.parity.shared::cta.b64 q, [%1], %2, %3;\n selp.u32 %0, 1, 0, q;\n}"
+                 : "=r"(ok) : "r"((uint32_t) __cvta_generic_to_shared(bar)), "r"(parity), "r"(kTryNs) : "memory");
     return ok != 0;
 }
-// Waits until the barrier's phase `parity` is over, at most kTeamWaits tries and not once the team is abandoned. A
-// wait that runs out abandons the team with kErrTraverseLimit. Uniform over the warp.
-constexpr int kTeamWaits = 1 << 24;
-__device__ __forceinline__ bool team_wait(unsigned long long *bar, unsigned parity, int *abandon, uint32_t *err) {
-    for (int k = 0; k < kTeamWaits; ++k) {
-        if (__all_sync(kFull, mbar_try_wait(bar, parity))) return true;
+// Waits until the barrier's phase `parity` is over, at most limit_ns and not once the team is abandoned. A
+// wait that runs out abandons the team with kErrTeamTimeout. Uniform over the warp.
+__device__ __forceinline__ bool team_wait(unsigned long long *bar, unsigned parity, int *abandon, uint32_t *err,
+                                          unsigned long long limit_ns) {
+    if (__all_sync(kFull, mbar_try_wait(bar, parity))) return true;
+    const unsigned long long t0 = global_timer_ns();
+    for (;;) {
         if (__any_sync(kFull, *(volatile int *) abandon != 0)) return false;
+        if (__any_sync(kFull, global_timer_ns() - t0 > limit_ns)) break;
+        if (__all_sync(kFull, mbar_try_wait(bar, parity))) return true;
     }
     if ((threadIdx.x & 31) == 0) {
-        atomicOr(err, (uint32_t) kErrTraverseLimit);
+        atomicOr(err, (uint32_t) kErrTeamTimeout);
         *(volatile int *) abandon = 1;
     }
     __syncwarp();
@@ -536,6 +546,7 @@ struct TeamSink {
     static constexpr int PAY = NodeLayout<ORDER>::PAY;
     TeamSmem<PAY, PART> &S;
     uint32_t *err;
+    unsigned long long limit_ns;  // of each wait
     int lane, n_bodies;
     int nfull = 0, npart = 0, npp = 0;
     int node_lists = 0, leaf_lists = 0;  // lists handed over
@@ -543,7 +554,7 @@ struct TeamSink {
 
     __device__ __forceinline__ NodeList *open_nodes() {
         const int slot = node_lists % kRing, turn = node_lists / kRing;
-        if (lost || (turn > 0 && !team_wait(&S.node_free[slot], (turn - 1) & 1, &S.abandon, err))) {
+        if (lost || (turn > 0 && !team_wait(&S.node_free[slot], (turn - 1) & 1, &S.abandon, err, limit_ns))) {
             lost = true;
             return nullptr;
         }
@@ -585,7 +596,7 @@ struct TeamSink {
     }
     __device__ __forceinline__ void hand_leaves(int count) {
         const int slot = leaf_lists % kLeafRing, turn = leaf_lists / kLeafRing;
-        if (lost || (turn > 0 && !team_wait(&S.leaf_free[slot], (turn - 1) & 1, &S.abandon, err))) {
+        if (lost || (turn > 0 && !team_wait(&S.leaf_free[slot], (turn - 1) & 1, &S.abandon, err, limit_ns))) {
             lost = true;
             return;
         }
@@ -887,7 +898,8 @@ __global__ void __launch_bounds__(kTeamThreads, kTeamBlocks)
     bh_team_kernel(NodeArrays nodes, const int *__restrict__ num_nodes_p, const float4 *__restrict__ bodies, int n_bodies,
                    const float4 *__restrict__ targets, int n_targets, float G, float eps, float4 *__restrict__ acc,
                    unsigned long long *__restrict__ counts, uint32_t *__restrict__ err, const int4 *__restrict__ groups,
-                   const int *__restrict__ inst_root, unsigned long long *__restrict__ inst_counts) {
+                   const int *__restrict__ inst_root, unsigned long long *__restrict__ inst_counts,
+                   unsigned long long wait_limit_ns) {
     constexpr int PAY = NodeLayout<ORDER>::PAY;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     TeamSmem<PAY, PART> &S = *reinterpret_cast<TeamSmem<PAY, PART> *>(smem_raw);
@@ -927,14 +939,14 @@ __global__ void __launch_bounds__(kTeamThreads, kTeamBlocks)
         const uint32_t full = __ballot_sync(kFull, valid);
         float lo[3], hi[3];
         target_box(p, valid, lo, hi);
-        TeamSink<ORDER, PART> sink{S, err, lane, n_bodies};
+        TeamSink<ORDER, PART> sink{S, err, wait_limit_ns, lane, n_bodies};
         walk(sink, nodes, num_nodes, root, full, lo, hi, S.tpos, S.stack, S.mixed_node, S.mixed_mask,
              walk_rounds(num_nodes), lanemask_lt(), lane, err);
         sink.finish();
     } else if (warp == 1) {
         for (int q = 0;; ++q) {
             const int slot = q % kRing;
-            if (!team_wait(&S.node_ready[slot], (q / kRing) & 1, &S.abandon, err)) break;
+            if (!team_wait(&S.node_ready[slot], (q / kRing) & 1, &S.abandon, err, wait_limit_ns)) break;
             const NodeList &l = S.nodes[slot];
             const int n = l.count;
             if (n < 0) break;
@@ -953,7 +965,7 @@ __global__ void __launch_bounds__(kTeamThreads, kTeamBlocks)
     } else {
         for (int q = warp - 2;; q += kLeafSets) {
             const int slot = q % kLeafRing;
-            if (!team_wait(&S.leaf_ready[slot], (q / kLeafRing) & 1, &S.abandon, err)) break;
+            if (!team_wait(&S.leaf_ready[slot], (q / kLeafRing) & 1, &S.abandon, err, wait_limit_ns)) break;
             const LeafList &l = S.leaf[slot];
             const int n = l.count;
             if (n < 0) break;
@@ -1041,6 +1053,7 @@ struct LaunchArgs {
     int64_t ngroups;
     const int *inst_root;
     unsigned long long *inst_counts;
+    unsigned long long wait_limit_ns = kTeamWaitNs;
 };
 
 // The team kernel's dynamic shared memory is enabled on first use per device.
@@ -1057,7 +1070,7 @@ void launch_team(const LaunchArgs &a, int device) {
     }
     kernel<<<(unsigned) a.ngroups, kTeamThreads, smem, a.s>>>(*a.nodes, a.num_nodes, a.bodies, a.n_bodies, a.targets,
                                                               a.nt, a.G, a.eps, a.acc, a.counts, a.err, a.gtab,
-                                                              a.inst_root, a.inst_counts);
+                                                              a.inst_root, a.inst_counts, a.wait_limit_ns);
 }
 
 template<int ORDER, bool EPS0, int THREADS, int PART>
@@ -1117,6 +1130,60 @@ int current_sm_count() {
 int64_t traverse_resident_warps(int device) {
     return std::max(std::max(max_resident_warps<1, false>(device), max_resident_warps<1, true>(device)),
                     std::max(max_resident_warps<2, false>(device), max_resident_warps<2, true>(device)));
+}
+
+// The tree is a chain of `rounds` internal nodes, opened by every target, whose left children are accepted by every
+// target: the walk takes one round per link (400 ns or more: two dependent loads and the classification) and
+// opens no leaf, so the six leaf warps wait for its whole length. The node warp and the walker see the team
+// abandoned at their next wait; the walk itself runs on to its end.
+cudaError_t team_timeout_selftest(unsigned long long wait_limit_ns, uint32_t *err_word) {
+    wait_limit_ns = std::min<unsigned long long>(wait_limit_ns, 100000000ull);
+    const int rounds = (int) (wait_limit_ns / 100), num_nodes = 2 * rounds + 1;
+    const std::unique_ptr<float4[]> mac(new (std::nothrow) float4[num_nodes]);
+    const std::unique_ptr<int2[]> link(new (std::nothrow) int2[num_nodes]);
+    if (!mac || !link) return cudaErrorMemoryAllocation;
+    for (int c = 0; c < num_nodes; ++c) {
+        const bool open = c % 2 == 0 && c + 2 < num_nodes;
+        mac[c] = make_float4(0.f, 0.f, 0.f, open ? FLT_MAX : 0.f);
+        link[c] = open ? make_int2(c + 2, -1) : make_int2(0, 1);
+    }
+    NodeArrays nodes;
+    float4 *bodies = nullptr, *acc = nullptr;
+    int *count = nullptr;
+    uint32_t *err = nullptr;
+    cudaError_t e = cudaSuccess;
+    auto alloc = [&](void **p, size_t bytes) {
+        if (e == cudaSuccess) e = cudaMalloc(p, bytes);
+        if (e == cudaSuccess) e = cudaMemset(*p, 0, bytes);
+    };
+    alloc((void **) &nodes.mac, num_nodes * sizeof(float4));
+    alloc((void **) &nodes.link, num_nodes * sizeof(int2));
+    alloc((void **) &nodes.pay, num_nodes * sizeof(float4));
+    alloc((void **) &bodies, 32 * sizeof(float4));
+    alloc((void **) &acc, 32 * sizeof(float4));
+    alloc((void **) &count, sizeof(int));
+    alloc((void **) &err, sizeof(uint32_t));
+    auto copy = [&](void *dst, const void *src, size_t bytes) {
+        if (e == cudaSuccess) e = cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice);
+    };
+    copy(nodes.mac, mac.get(), num_nodes * sizeof(float4));
+    copy(nodes.link, link.get(), num_nodes * sizeof(int2));
+    copy(count, &num_nodes, sizeof(int));
+    if (e == cudaSuccess) {
+        int device = 0;
+        cudaGetDevice(&device);
+        LaunchArgs a{&nodes, count, bodies, 32, bodies, 32, 1, 1.f, 1.f, acc, nullptr, nullptr, err, nullptr,
+                     nullptr, 1, nullptr, nullptr};
+        a.wait_limit_ns = wait_limit_ns;
+        launch_team<1, false, 64>(a, device);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaDeviceSynchronize();
+    if (e == cudaSuccess) e = cudaMemcpy(err_word, err, sizeof(uint32_t), cudaMemcpyDeviceToHost);
+    for (void *p: {(void *) nodes.mac, (void *) nodes.link, (void *) nodes.pay, (void *) bodies, (void *) acc,
+                   (void *) count, (void *) err})
+        if (p) cudaFree(p);
+    return e;
 }
 
 bool traversal_shape_valid(int threads, int slab) { return (threads == 128 || threads == 256) && (slab == 32 || slab == 64); }
