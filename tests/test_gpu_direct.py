@@ -82,3 +82,34 @@ def test_energy(nb, n, eps):
         kinetic, potential = s.energy()
     assert abs(kinetic - k) <= 1e-14 * k
     assert abs(potential + 0.5 * u) <= 1e-14 * max(u, 1e-300)
+
+
+@pytest.mark.parametrize("precision", [32, 64])
+def test_infinite_distances_add_zero(nb, precision):
+    """A source at infinity along one axis leaves the other axes' sums alone, a target there has none along
+    them, and infinite softening leaves no sum at all."""
+    import torch
+
+    pm, vel = nb.scenarios.plummer(300, seed=9)
+    far = np.array([[np.inf, 0.25, -0.5, 1.0]], np.float32)
+
+    def sums(bodies, eps, targets=pm[:40]):
+        b, t = torch.from_numpy(bodies).cuda(), torch.from_numpy(targets.copy()).cuda()
+        acc = torch.zeros(len(targets), 4 if precision == 32 else 3, device="cuda",
+                          dtype=torch.float32 if precision == 32 else torch.float64)
+        torch.cuda.synchronize()
+        with nb.NaiveSolver(None, nb.Gravity(1.0, eps)) as s:
+            s.direct_device(len(bodies), b.data_ptr(), len(targets), t.data_ptr(), acc.data_ptr(), precision)
+            s.synchronize()
+        return acc.cpu().numpy()[:, :3]
+
+    eps = float(np.float32(1e-4))
+    ref, size = reference(pm, pm[:40], eps)
+    got = sums(np.concatenate([pm[:100], far, pm[100:]]), eps)
+    assert np.isnan(got[:, 0]).all()
+    assert (np.abs(got[:, 1:] - ref[:, 1:]) <= (4e-6 if precision == 32 else 2e-14) * size[:, 1:]).all()
+    got = sums(pm, eps, far)
+    assert np.isnan(got[0, 0]) and (got[0, 1:] == 0).all()
+    assert (sums(pm, np.inf) == 0).all()
+    with nb.NaiveSolver(pm, nb.Gravity(1.0, np.inf), vel) as s:
+        assert s.energy()[1] == 0.0
