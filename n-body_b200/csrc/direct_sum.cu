@@ -139,9 +139,11 @@ __global__ void __launch_bounds__(kThreads) direct_f32_kernel(const float4 *__re
     }
 }
 
-// 1 / sqrt(x) of a normal x > 0 in FP64: the hardware's seed (relative error below 2^-19) and one step of
-// Householder's third-order iteration, y (1 + h / 2 + 3 h^2 / 8) with h = 1 - x y^2, whose own error is below
-// 2^-57: 5 FP64 operations, against a square root and a divide of some 20 each.
+// 1 / sqrt(x) of a normal x > 0 in FP64: the hardware's seed y and one step of Householder's third-order
+// iteration, y (1 + h / 2 + 3 h^2 / 8) with h = 1 - x y^2: 5 FP64 operations, against a square root and a
+// divide of some 20 each. The first term left out is 5/16 h^3. |h| is below 2^-19 (2^-19.04 at most over every
+// high word of [1, 4), on which alone the seed depends), so that the term is below 2^-58; y^2 is exact (20
+// mantissa bits), and the last operation's rounding is all that counts.
 // FAR: x may be infinite, where the root is 0 and h a NaN. The three instructions that tell cost 6 % (1.34 -> 1.42 ms
 // for 4,096 targets x 2^18 bodies), so only tiles that can need them take them.
 template<bool FAR>

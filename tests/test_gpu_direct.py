@@ -113,3 +113,48 @@ def test_infinite_distances_add_zero(nb, precision):
     assert (sums(pm, np.inf) == 0).all()
     with nb.NaiveSolver(pm, nb.Gravity(1.0, np.inf), vel) as s:
         assert s.energy()[1] == 0.0
+
+
+# One term each, so that the reciprocal root's error shows. With u = 2^-53, differences to a body at the origin
+# exact and G = 1: |r|^2 + eps carries 4 u, its root 2 u and u of its own; the force's factor takes three times
+# that, three products and the product with the difference, 13 u in all (14 u allowed); the potential the root, two
+# products and one sum, 6 u (7 u allowed). The reference is in extended precision.
+ULP = np.longdouble(2.0) ** -53
+
+
+@pytest.mark.parametrize("eps", [0.0, 1e-4])
+def test_fp64_force_term(nb, eps):
+    import torch
+
+    rng = np.random.default_rng(11)
+    nt = 20000
+    d = rng.standard_normal((nt, 3))
+    t = np.zeros((nt, 4), np.float32)
+    t[:, :3] = d / np.linalg.norm(d, axis=1)[:, None] * 10.0 ** rng.uniform(-6, 6, (nt, 1))
+    source = np.array([[0.0, 0.0, 0.0, 0.37]], np.float32)
+    eps = np.float32(eps)
+    b, tt = torch.from_numpy(source).cuda(), torch.from_numpy(t).cuda()
+    acc = torch.zeros(nt, 3, device="cuda", dtype=torch.float64)
+    torch.cuda.synchronize()
+    with nb.NaiveSolver(None, nb.Gravity(1.0, float(eps))) as s:
+        s.direct_device(1, b.data_ptr(), nt, tt.data_ptr(), acc.data_ptr(), 64)
+        s.synchronize()
+    x = t[:, :3].astype(np.longdouble)
+    r2 = (x * x).sum(1) + np.longdouble(eps)
+    ref = -x * (np.longdouble(source[0, 3]) / (r2 * np.sqrt(r2)))[:, None]
+    assert (np.abs(acc.cpu().numpy().astype(np.longdouble) - ref) <= 14 * ULP * np.abs(ref)).all()
+
+
+@pytest.mark.parametrize("eps", [0.0, 1e-4])
+def test_fp64_potential_term(nb, eps):
+    rng = np.random.default_rng(12)
+    eps = np.float32(eps)
+    with nb.NaiveSolver(None, nb.Gravity(1.0, float(eps))) as s:
+        for k in range(60):
+            pm = np.zeros((2, 4), np.float32)
+            pm[1, :3] = rng.standard_normal(3) * 10.0 ** rng.uniform(-6, 6)
+            pm[:, 3] = rng.uniform(0.1, 2.0, 2)
+            s.set_bodies(pm)
+            x = pm.astype(np.longdouble)
+            ref = -x[0, 3] * x[1, 3] / np.sqrt((x[1, :3] ** 2).sum() + np.longdouble(eps))
+            assert abs(np.longdouble(s.energy()[1]) - ref) <= 7 * ULP * abs(ref)
