@@ -78,6 +78,7 @@ struct nb_ctx {
     std::vector<int64_t> inst_start, inst_size;
     int *inst_of = nullptr, *inst_root = nullptr;
     float *inst_theta2 = nullptr;
+    float batch_theta = 0.f;  // the instances' mean
     uint32_t *inst_box = nullptr;  // 6 order-preserving uints per instance (min.xyz, ~max.xyz)
     int inst_bbox_slices = 1;      // blocks per instance of the box reduction
     int2 *inst_range = nullptr;
@@ -486,7 +487,8 @@ int force_pass_batch(nb_ctx *ctx, Marks &mk) {
     mk.mark(kTraverse);
     cudaMemsetAsync(ctx->inst_counts, 0, (size_t) 2 * ctx->num_inst * sizeof(unsigned long long), s);
     launch_bh_traverse(ctx->cfg.order, ctx->nodes, ctx->tw.num_nodes, ctx->pos, n, ctx->pos, n,
-                       ctx->cfg.max_leaf_size, ctx->cfg.G, ctx->cfg.epsilon, ctx->acc, ctx->counts, ctx->trav, ctx->err, s, ctx->groups, ctx->ngroups,
+                       TreeShape{ctx->cfg.max_leaf_size, ctx->batch_theta, ctx->num_inst}, ctx->cfg.G,
+                       ctx->cfg.epsilon, ctx->acc, ctx->counts, ctx->trav, ctx->err, s, ctx->groups, ctx->ngroups,
                        ctx->inst_root, ctx->inst_counts);
     ctx->have_tree = true;
     ctx->acc_is_bh = true;
@@ -549,7 +551,8 @@ int force_pass(nb_ctx *ctx, Marks &mk) {
     mk.mark(kTraverse);
     // a sharded context evaluates only its slice of the Morton-ordered targets
     launch_bh_traverse(ctx->cfg.order, ctx->nodes, ctx->tw.num_nodes, ctx->pos, n, ctx->pos + first, count,
-                       ctx->cfg.max_leaf_size, ctx->cfg.G, ctx->cfg.epsilon, ctx->acc + first, ctx->counts, ctx->trav, ctx->err, s);
+                       TreeShape{ctx->cfg.max_leaf_size, ctx->cfg.theta, 1}, ctx->cfg.G, ctx->cfg.epsilon,
+                       ctx->acc + first, ctx->counts, ctx->trav, ctx->err, s);
     ctx->have_tree = true;
     ctx->acc_is_bh = true;
     if (ctx->timing) ctx->times.launches += launches_per_pass(ctx, need_bbox, false);
@@ -1076,6 +1079,7 @@ static int build_batch_tables(nb_ctx *ctx, int32_t count, const int64_t *sizes, 
     std::vector<int2> range((size_t) count);
     std::vector<int> group_first((size_t) count);
     std::vector<float> theta2((size_t) count);
+    double theta_sum = 0.0;
     std::vector<uint32_t> hist(2 * 256, 0);
     ctx->inst_start.resize(count);
     ctx->inst_size.assign(sizes, sizes + count);
@@ -1087,6 +1091,7 @@ static int build_batch_tables(nb_ctx *ctx, int32_t count, const int64_t *sizes, 
         ngroups += (sizes[k] + 31) / 32;
         const float th = thetas ? thetas[k] : ctx->cfg.theta;
         theta2[k] = th * th;  // the reference compares against theta * theta in float
+        theta_sum += th;
         hist[k & 255] += (uint32_t) sizes[k];
         hist[256 + (k >> 8)] += (uint32_t) sizes[k];
         start += sizes[k];
@@ -1140,6 +1145,7 @@ static int build_batch_tables(nb_ctx *ctx, int32_t count, const int64_t *sizes, 
     NB_TRY(cudaMemcpyAsync(ctx->inst_hist, hist.data(), hist.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, s),
            "copy");
     ctx->num_inst = count;
+    ctx->batch_theta = (float) (theta_sum / count);
     ctx->ngroups = ngroups;
     ctx->inst_passes = passes;
     // host vectors are released on return: wait for the copies out of them

@@ -332,14 +332,20 @@ int64_t traverse_resident_warps(int device);
 // groups (optional): one int4 (first target, target count <= 32, instance, 0) per warp task; the
 // traversal of a group starts at inst_root[instance]. Without groups, targets are cut into
 // consecutive groups of 32 that start at node 0. inst_counts (optional, with groups): per instance,
-// (particle-particle, node-particle) interaction counts are added at [2 * instance + {0, 1}]. leaf:
-// the tree's largest leaf (it moves the line between the traversal's two forms, nothing else).
+// (particle-particle, node-particle) interaction counts are added at [2 * instance + {0, 1}].
+// What the line between the traversal's two forms depends on (nothing else does): the largest leaf, the
+// opening angle (of a batch, the mean) and the number of trees.
+struct TreeShape {
+    int leaf = 1;
+    float theta = 0.f;
+    int trees = 1;
+};
 // Self-test of the team form's bounded waits: one group whose walk hands no leaf list over for several
 // times wait_limit_ns (100 ms at most), so that the warps waiting for one give up. The error word it
 // leaves is returned (kErrTeamTimeout expected).
 cudaError_t team_timeout_selftest(unsigned long long wait_limit_ns, uint32_t *err_word);
 void launch_bh_traverse(int order, const NodeArrays &nodes, const int *num_nodes, const float4 *bodies, int64_t n_bodies,
-                        const float4 *targets, int64_t n_targets, int leaf, float G, float eps, float4 *acc,
+                        const float4 *targets, int64_t n_targets, TreeShape shape, float G, float eps, float4 *acc,
                         unsigned long long *counts, TraverseWorkspace &ws, uint32_t *err, cudaStream_t s,
                         const int4 *groups = nullptr, int64_t num_groups = 0, const int *inst_root = nullptr,
                         unsigned long long *inst_counts = nullptr);

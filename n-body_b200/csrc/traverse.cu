@@ -40,6 +40,7 @@
 #include <algorithm>
 #include <cfloat>
 #include <climits>
+#include <cmath>
 #include <memory>
 #include <new>
 
@@ -1025,15 +1026,32 @@ int resident_warps(int device) {
 }
 
 // Launches of at most this many groups run one team of warps per group, larger ones one warp per
-// group. The team form has one walking warp in eight, so it loses where the groups alone fill the
-// GPU; larger leaves shift work from the walk to the leaf warps and the line with it. Measured
-// (warp form over team form, traversal time, orders 1 and 2, theta 0.3 to 0.65, Plummer and ball):
-// leaf 8: 2.0-3.4 at 16k bodies, 1.1-1.6 at 49k, 0.9-1.15 at 65k; leaf 16: 1.06-1.8 at 65k,
-// 0.86-1.4 at 98k; leaf 32: 1.03-1.7 at 131k, 0.84-1.3 at 196k; leaf 64: 1.1-1.5 at 196k,
-// 0.98-1.2 at 262k. Leaves above 64 bodies give too few lists to share out: always one warp.
-int64_t team_groups(int device, int leaf) {
+// group. The team form has one walking warp in eight and four blocks per SM, so it loses where the groups alone
+// fill the GPU. The line, in groups per SM:
+//   - one wave of teams (four) always gains;
+//   - above, larger leaves shift work from the walk to the leaf warps, and the line with it; theta above 0.5
+//     opens fewer leaves (the exponent fits theta 0.7 and 1);
+//   - a slice of a larger set (a shard) has no sparse outskirts, whose few long groups hold one warp up
+//     longest, and a deeper tree to walk;
+//   - trees of few leaves give a group hardly more to do than a team's start and end cost.
+// Measured, time with one warp over time with teams (g: groups per SM):
+//   whole sets at theta 0.5, Plummer and ball: leaf 1 1.07-1.09 at g 6, 0.96-1.07 at 8; leaf 8 1.02-1.15 at 10,
+//     0.83-0.87 at 14; leaf 16 1.03-1.10 at 14, 0.96-0.99 at 18; leaf 32 0.98-1.10 at 30; leaf 64 0.99-1.07 at 54;
+//   theta 0.7: leaf 8 1.00-1.08 at 10, 0.90-0.96 at 12; leaf 16 1.07-1.14 at 12, 0.95 at 14; leaf 32 1.04-1.18
+//     at 18, 0.86-0.89 at 24; theta 1: leaf 8 0.99-1.12 at 8; leaf 16 0.97-1.07 at 10;
+//   slices of 300,000 to 2^22 bodies: leaf 8 0.94-1.02 at 9; leaf 16 1.01-1.26 at 10.6, 0.83-1.05 at 13; leaf 32
+//     0.93-1.19 at 17; leaf 64 0.93-1.17 at 32;
+//   batches at leaf 16: instances of 33 to 200 bodies 1.05-1.15 at 3, 0.80-0.86 at 6, 0.5 at 18; of 500 1.5 at 3,
+//     0.93 at 6; of 1000 1.09 at 6, 0.85 at 12; of 2500 1.14 at 12, 0.98 at 18; at leaf 64 1000 0.83 at 6, 2500
+//     1.03 at 6, 0.81 at 12, 8000 1.04 at 29.
+// Leaves above 64 bodies run one warp per group, although teams gain there too (1.15-3.2 for leaves of 65 to 256
+// at theta 0.5 and up to 50 groups per SM, 1.04-1.7 for leaves of 1000).
+int64_t team_groups(int device, int leaf, float theta, int64_t tree_bodies, bool slice) {
     if (leaf > 64) return 0;
-    return (int64_t) sm_count(device) * (24 + 3 * leaf) / 4;
+    const double opened = theta > 0.5f ? std::pow(0.5 / theta, 1.75) : 1.0;
+    const double most = 6.0 + 0.75 * leaf * opened * (slice ? 0.45 : 1.0);
+    const double few = std::min(1.0, (double) tree_bodies / (128.0 * leaf));
+    return (int64_t) (sm_count(device) * (4.0 + (most - 4.0) * few * few));
 }
 
 struct LaunchArgs {
@@ -1042,7 +1060,8 @@ struct LaunchArgs {
     const float4 *bodies;
     int n_bodies;
     const float4 *targets;
-    int nt, leaf;
+    int nt;
+    TreeShape shape;
     float G, eps;
     float4 *acc;
     unsigned long long *counts;
@@ -1078,7 +1097,9 @@ void launch_variant(const LaunchArgs &a) {
     constexpr int kWarps = THREADS / 32;
     int device = 0;
     cudaGetDevice(&device);
-    if (a.ngroups <= team_groups(device, a.leaf)) {
+    // a slice holds at most a quarter of its set
+    const bool slice = a.n_bodies / 4 >= a.nt;
+    if (a.ngroups <= team_groups(device, a.shape.leaf, a.shape.theta, a.n_bodies / std::max(a.shape.trees, 1), slice)) {
         launch_team<ORDER, EPS0, PART>(a, device);
         return;
     }
@@ -1172,7 +1193,7 @@ cudaError_t team_timeout_selftest(unsigned long long wait_limit_ns, uint32_t *er
     if (e == cudaSuccess) {
         int device = 0;
         cudaGetDevice(&device);
-        LaunchArgs a{&nodes, count, bodies, 32, bodies, 32, 1, 1.f, 1.f, acc, nullptr, nullptr, err, nullptr,
+        LaunchArgs a{&nodes, count, bodies, 32, bodies, 32, TreeShape(), 1.f, 1.f, acc, nullptr, nullptr, err, nullptr,
                      nullptr, 1, nullptr, nullptr};
         a.wait_limit_ns = wait_limit_ns;
         launch_team<1, false, 64>(a, device);
@@ -1189,12 +1210,12 @@ cudaError_t team_timeout_selftest(unsigned long long wait_limit_ns, uint32_t *er
 bool traversal_shape_valid(int threads, int slab) { return (threads == 128 || threads == 256) && (slab == 32 || slab == 64); }
 
 void launch_bh_traverse(int order, const NodeArrays &nodes, const int *num_nodes, const float4 *bodies, int64_t n_bodies,
-                        const float4 *targets, int64_t n_targets, int leaf, float G, float eps, float4 *acc,
+                        const float4 *targets, int64_t n_targets, TreeShape shape, float G, float eps, float4 *acc,
                         unsigned long long *counts, TraverseWorkspace &ws, uint32_t *err, cudaStream_t s,
                         const int4 *gtab, int64_t ngroups, const int *inst_root, unsigned long long *inst_counts) {
     if (n_targets <= 0) return;
     if (!gtab) ngroups = (n_targets + 31) / 32;
-    const LaunchArgs a{&nodes, num_nodes, bodies, (int) n_bodies, targets, (int) n_targets, leaf, G, eps, acc, counts, &ws,
+    const LaunchArgs a{&nodes, num_nodes, bodies, (int) n_bodies, targets, (int) n_targets, shape, G, eps, acc, counts, &ws,
                        err, s, gtab, ngroups, inst_root, inst_counts};
     const bool ok = traversal_shape_valid(ws.threads, ws.slab);
     const int threads = ok ? ws.threads : 256, part = ok ? ws.slab : 64;

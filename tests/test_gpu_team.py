@@ -30,3 +30,27 @@ def test_team_and_single_warp_forms_agree(nb, n, order, leaf, eps, slab):
         per = s.instance_counts()
     assert np.array_equal(alone, batch[:n])
     assert (counts["particle_particle"], counts["node_particle"]) == tuple(int(x) for x in per[0])
+
+
+@pytest.mark.parametrize("n,order,leaf,eps,slab,theta", [
+    (40_001, 2, 8, 1e-4, 64, 0.5),  # sizes near the largest that run teams: full rings, a walker that waits
+    (60_007, 2, 16, 0.0, 64, 0.5),
+    (60_007, 1, 16, 1e-4, 32, 0.3),
+    (100_003, 2, 64, 0.0, 32, 0.5),
+    (100_003, 1, 64, 1e-5, 64, 0.3),
+])
+def test_forms_agree_in_full_rings(nb, n, order, leaf, eps, slab, theta):
+    pm, _ = nb.scenarios.plummer(n, seed=n)
+    big, _ = nb.scenarios.uniform_ball(300_000, seed=7)
+    cls = nb.LinearBVHSolver if order == 1 else nb.QuadrupoleLinearBVHSolver
+    kw = dict(theta=theta, max_leaf_size=leaf)
+    with cls(pm, nb.Gravity(1.0, eps), **kw) as s:
+        s.traversal_shape = (256, slab)
+        alone, counts = s.update_accelerations(), s.counts()
+    with cls(None, nb.Gravity(1.0, eps), **kw) as s:
+        s.traversal_shape = (256, slab)
+        s.set_instances([n, len(big)], np.concatenate([pm, big]))
+        batch = s.update_accelerations()
+        per = s.instance_counts()
+    assert np.array_equal(alone, batch[:n])
+    assert (counts["particle_particle"], counts["node_particle"]) == tuple(int(x) for x in per[0])
