@@ -17,7 +17,7 @@
 //                     and the number of final nodes starting at each body position
 //   scan kernels      exclusive prefix over body positions of those counts: the preorder index of
 //                     the final leaf starting at each position
-//   summarize_kernel  one block per 1024 or 4096 Karras nodes, one thread per final internal node with
+//   summarize_kernel  one block per 128 to 4096 Karras nodes (climb_nodes), one thread per final internal node with
 //                     leaf children: sequential leaf summaries over the leaf's bodies, then a climb in
 //                     which the second child to arrive summarises the parent (CenterOfMassSummary.h:30-55,
 //                     BoundingBoxSummary.h:30-68, MultipoleMassSummary.h:37-97; the leaf moment
@@ -32,6 +32,7 @@
 //                     at f (a chain of left children), the larger ones; a leaf starting at f comes
 //                     after that whole chain.
 #include <algorithm>
+#include <type_traits>
 #include <cfloat>
 
 #include "nb_internal.cuh"
@@ -643,10 +644,7 @@ __device__ __forceinline__ Summ<ORDER> combine(const TreeWorkspace &tw, const Su
 // Karras indices in [first, last], so a node whose range lies in the block's index range is climbed
 // to by this block's threads alone: its arrivals are counted in shared memory and need block-scope
 // ordering only, a few hundred cycles instead of the device-scope arrival's round trips to L2.
-// 1024 nodes hold enough leaf parents for 128 threads at leaves of up to some 16 bodies; larger leaves
-// take 4096 (2^22 bodies at leaf 64, octupole: 0.77 ms with 1024).
 constexpr int kClimbThreads = 128;
-constexpr int kClimbSmall = 1024, kClimbLarge = 4096;
 
 template<int NODES>
 struct ClimbSmem {
@@ -796,10 +794,10 @@ __device__ void write_records(int n, const TreeWorkspace &tw, uint32_t *err, con
 // lists its nodes with leaf children (then its final nodes) first, so that threads climb and do not idle
 // over the nodes in between. The whole tree is one leaf when n == 1, or when the root is not
 // splittable (n <= maxLeafSize or every code equal): the first block's first thread writes it.
-// Cold-cache times, before (device-scope arrivals at every level, records on the chain, a list of leaf
-// parents made by karras_kernel) and now: 1,023 bodies 66 and 47 us, 10,000 (monopole) 46 and 52 us, 2^20 bodies 112
-// and 145 us with karras_kernel 73 and 46 us, 9.3 million bodies in 256 instances 2.65 and 0.77 ms; four launches
-// and clears fewer per build.
+// Whole build (CUDA events), before (device-scope arrivals at every level, records on the chain, a list of leaf
+// parents made by karras_kernel) and now: 1,500 bodies 87 and 71 us, 10,000 (monopole) 75 and 59, 100,000 130 and
+// 117, 2^20 189 and 182, 2^22 (leaf 16) 483 and 431, 9.2 million in 256 instances 1,203 and 1,085 us; 2^22 at leaf 64
+// 319 and 367 us, octupole 415 and 523: there the chain of levels is hidden and a block's last climbs are not.
 template<int ORDER, int NODES, class Records>
 __global__ void __launch_bounds__(kClimbThreads) summarize_kernel(const float4 *__restrict__ bodies, int n, TreeWorkspace tw,
                                                                   uint32_t *err, Records rec) {
@@ -834,14 +832,43 @@ __global__ void __launch_bounds__(kClimbThreads) summarize_kernel(const float4 *
         write_records<ORDER, NODES, Records>(n, tw, err, rec, lo + S.list[1][k]);
 }
 
+// Karras nodes per block of the climb. Larger blocks keep more of it inside; they also leave fewer blocks,
+// and a block's 128 threads take its leaf parents in turn. So the size grows with n, such that some 400 blocks or
+// more are left (twice as large for the octupole, whose records above the blocks cost more), up to a
+// number of leaf parents that keeps the threads busy. A set that one block holds, with a leaf parent or two per
+// thread, takes one block. Whole build, us, 128 / 256 / 512 / 1024 / 2048 / 4096 nodes per block, quadrupole unless stated:
+//   1,000 bodies    leaf 2   73 / 73 / 82 / 83 / 81 / 84, leaf 16 65 / 65 / 65 / 47 / 47 / 47
+//   3,000           leaf 16  79 / 77 / 77 / 79 / 78 / 85, leaf 32 75 / - / - / 79 / 77 / 62
+//   20,000          leaf 1   114 / 130 / 145 / 172 / 280 / 483, leaf 16 106 / 107 / 112 / 111 / 122 / 148
+//   100,000         leaf 2   135 / 129 / 141 / 178 / 239 / 409, leaf 64 124 / 120 / 123 / 126 / 129 / 134
+//   300,000         leaf 1   212 / 212 / 192 / 228 / 326 / 558, leaf 16 183 / 149 / 131 / 133 / 141 / 174
+//   2^20            leaf 2   484 / 376 / 343 / 361 / 393 / 556, leaf 8 462 / 323 / 245 / 213 / 220 / 298,
+//                   leaf 16  446 / 312 / 232 / 198 / 181 / 226, octupole leaf 64 745 / 615 / 428 / 319 / 273 / 241
+//   2^22            leaf 16  1559 / 1007 / 684 / 501 / 430 / 465, leaf 64 1357 / 1050 / 754 / 556 / 434 / 385
+int climb_nodes(int n, int leaf, int order) {
+    if (n <= 4097 && n <= (int64_t) leaf * (n <= 1025 ? 256 : 100)) return n <= 1025 ? 1024 : n <= 2049 ? 2048 : 4096;
+    const int most = leaf <= 2 ? 512 : leaf <= 8 ? 1024 : leaf <= 16 ? 2048 : 4096;
+    int nodes = 128;
+    while (nodes < most && (int64_t) n >= 2 * (int64_t) nodes * (order >= 3 ? 192 : 384)) nodes *= 2;
+    return nodes;
+}
+
 template<int ORDER, class Records>
 void launch_summarize(const float4 *bodies, int n, int leaf, const TreeWorkspace &tw, uint32_t *err, cudaStream_t s,
                       const Records &rec) {
-    auto blocks = [n](int nodes) { return (unsigned) std::max(1, (n - 1 + nodes - 1) / nodes); };
-    if (leaf > 16)
-        summarize_kernel<ORDER, kClimbLarge, Records><<<blocks(kClimbLarge), kClimbThreads, 0, s>>>(bodies, n, tw, err, rec);
-    else
-        summarize_kernel<ORDER, kClimbSmall, Records><<<blocks(kClimbSmall), kClimbThreads, 0, s>>>(bodies, n, tw, err, rec);
+    auto launch = [&](auto nodes) {
+        constexpr int kNodes = decltype(nodes)::value;
+        const unsigned blocks = (unsigned) std::max(1, (n - 1 + kNodes - 1) / kNodes);
+        summarize_kernel<ORDER, kNodes, Records><<<blocks, kClimbThreads, 0, s>>>(bodies, n, tw, err, rec);
+    };
+    switch (climb_nodes(n, leaf, ORDER)) {
+        case 128: return launch(std::integral_constant<int, 128>());
+        case 256: return launch(std::integral_constant<int, 256>());
+        case 512: return launch(std::integral_constant<int, 512>());
+        case 1024: return launch(std::integral_constant<int, 1024>());
+        case 2048: return launch(std::integral_constant<int, 2048>());
+        default: return launch(std::integral_constant<int, 4096>());
+    }
 }
 
 // Karras topology, the final nodes per start position (tw.start is zero on entry) and their

@@ -1,5 +1,5 @@
-"""The tree build at the edges of its climb blocks (1024 and 4096 Karras nodes) and of its prefix scans (one kernel
-up to eight 2048-position tiles, two above): every node record bit-exact against the oracle."""
+"""The tree build at the edges of its climb blocks (128 to 4096 Karras nodes by size and leaf) and of its prefix
+scans (one kernel up to eight 2048-position tiles, two above): every node record bit-exact against the oracle."""
 import numpy as np
 import pytest
 
@@ -24,4 +24,21 @@ def test_dual_records_at_block_edges(nb, oracle, n, leaf):
     pm, _ = nb.scenarios.hernquist(n, seed=n)
     with dual_solver(nb, pm, leaf, 0.5) as s:
         s.update_accelerations()
+        check_dual_tree(nb, oracle, s, pm, leaf)
+
+
+@pytest.mark.parametrize("n,leaf", [(257, 1), (1027, 1), (1700, 17), (2050, 16), (4097, 41), (4098, 41), (98_303, 1), (98_305, 5), (200_003, 2), (400_001, 4), (800_003, 16),
+                                    (1_600_001, 32)])
+def test_records_by_block_size(nb, oracle, n, leaf):
+    pm, _ = nb.scenarios.plummer(n, seed=n)
+    with make_solver(nb, pm, order=2, leaf=leaf) as s:
+        s.update_accelerations_async()
+        check_tree(nb, oracle, s, pm, leaf, 2, 0.5)
+
+
+@pytest.mark.parametrize("n,leaf", [(49_153, 64), (100_003, 16), (200_001, 17), (400_001, 16), (800_003, 64)])
+def test_dual_records_by_block_size(nb, oracle, n, leaf):
+    pm, _ = nb.scenarios.hernquist(n, seed=n)
+    with dual_solver(nb, pm, leaf, 0.5) as s:
+        s.update_accelerations_async()
         check_dual_tree(nb, oracle, s, pm, leaf)
