@@ -395,7 +395,7 @@ int dual_traverse(nb_ctx *ctx, int64_t n, int64_t first, int64_t count, cudaStre
     NearPool &np = ctx->dws.near;
     for (int attempt = 0;; ++attempt) {
         launch_dual_traverse(ctx->dnodes, ctx->tw.num_nodes, ctx->pos, n, ctx->cfg.G, ctx->cfg.epsilon,
-                             ctx->cfg.theta, ctx->acc, ctx->counts, ctx->dws, ctx->err, s, first, first + count);
+                             ctx->cfg.theta, ctx->cfg.max_leaf_size, ctx->acc, ctx->counts, ctx->dws, ctx->err, s, first, first + count);
         unsigned long long *h = ctx->host_scratch;
         SpillPool &sp = ctx->dws.spill;
         NB_TRY(cudaMemcpyAsync(h, np.counters, 4 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s),

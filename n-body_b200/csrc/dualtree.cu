@@ -1568,7 +1568,20 @@ __global__ void __launch_bounds__(kNearThreads, 8) near_kernel(DualNodes nodes, 
 
 }  // namespace
 
+// Passive nodes of at most this many bodies below a larger parent are handed to the second kernel, which balances
+// them over the whole GPU: 64 bodies in small sets (more would leave the first kernel's tasks too large),
+// sqrt(n) / 2 above (fewer nodes, longer lists each), less for leaves below 64, whose deeper subtrees cost more. Whole traversal, ms, 64 / 128 / 181 / 256:
+//   leaf 8  theta 0.6  131,072: 20.7 (64) / 23.6 (181), 250,000: 51.0 (64) / 51.8 (250)
+//   leaf 16 theta 0.6  131,072:  9.4 /  9.6 / 10.4 / 11.6, 180,000: 14.6 / 14.1 / 14.3 / 15.3, 250,000: 22.8 / 21.4 / 21.2 / 21.8
+//   leaf 32 theta 0.5   90,000:  4.9 /  4.8 /  5.4 /  6.2, 131,072:  7.1 /  6.8 /  7.2 /  8.0, 250,000: 17.7 / 15.5 / 15.2 / 15.3
+//   leaf 64 theta 0.4   90,000:  4.5 /  4.3 /  4.4 /  4.9, 131,072:  7.3 /  6.7 /  6.7 /  7.1, 500,000: 47.2 / 40.4 / 38.1 / 37.3
+// and, 256 / 512 / 1024: 10^6 at theta 0.5 58.7 / 56.2 / 62.1, 2^22 at 0.4 365 / 346 / 341; 6 and 9 million bodies
+// as with n / 4096.
 constexpr int64_t kSmallDual = 131072;
+static int frontier_bodies(int64_t n, int leaf) {
+    if (n < kSmallDual) return 64;
+    return std::max(64, (int) (0.5 * std::sqrt((double) n * std::min(leaf, 64) / 64.0)));
+}
 
 // Near-field grid: the resident blocks, never more than the walk stacks allocated (one per warp).
 unsigned near_grid(const DualWorkspace &ws) {
@@ -1577,7 +1590,7 @@ unsigned near_grid(const DualWorkspace &ws) {
 }
 
 void launch_dual_traverse(const DualNodes &nodes, const int *num_nodes, const float4 *bodies, int64_t n, float G,
-                          float eps, float theta, float4 *acc, unsigned long long *counts, DualWorkspace &ws,
+                          float eps, float theta, int leaf, float4 *acc, unsigned long long *counts, DualWorkspace &ws,
                           uint32_t *err, cudaStream_t s, int64_t t_lo, int64_t t_hi) {
     if (n <= 0) return;
     const int lo = (int) std::max<int64_t>(0, std::min(t_lo, n)), hi = (int) std::max<int64_t>(lo, std::min(t_hi, n));
@@ -1587,15 +1600,11 @@ void launch_dual_traverse(const DualNodes &nodes, const int *num_nodes, const fl
     cudaMemsetAsync(ws.spill.head, 0xFF, (size_t) ws.spill.head_cap * sizeof(int), s);
     cudaMemsetAsync(ws.spill.counters, 0, 4 * sizeof(unsigned long long), s);
     load_balanced_break_kernel<<<1, 512, 0, s>>>(nodes, num_nodes, ws.roots, ws.num_roots, err);
-    // passive nodes of at most `frontier` bodies below a larger parent are handed to the second
-    // kernel, which balances them over the whole GPU
-    // Measured (whole traversal, theta 0.4 and 0.5, frontier 64 / 128 / 256 / 512 / 1024): 60,001 bodies
-    // 2.94-3.23 / 2.79-3.41 / 3.5-4.4 ms; 250,000: 17.6-19.7 / 15.6-16.8 / 15.2-16.3 / 18.8-19.9 ms; 10^6 at 0.5:
-    // 58.7 (256) / 56.2 / 62.1 ms; 2^22 at 0.4: 365 (256) / 346 / 341 ms.
-    const int frontier = n < kSmallDual ? 64 : (int) (0.5 * std::sqrt((double) n));
+    const int frontier = frontier_bodies(n, leaf);
     // Few units leave warps idle and the largest one sets the near field's time: half-size units (two
-    // replicas of each target) below kSmallDual bodies. 60,001 bodies: 3.24 -> 2.82 ms and 3.00 -> 2.56 ms;
-    // 250,000: 17.6 -> 18.1 ms.
+    // replicas of each target) below kSmallDual bodies. Whole traversal, ms, units of 16 / 32: 60,001 bodies 2.85 /
+    // 3.14 (leaf 32) and 2.54 / 2.93 (leaf 64), 90,000 4.91 / 4.87 and 4.55 / 4.82, 131,072 7.35 / 7.07 and 7.38 /
+    // 7.28, 250,000 18.1 / 17.7 and 20.3 / 19.8; leaves of 16 fill no larger unit.
     ws.near.unit = n < kSmallDual ? 16 : 32;
     dual_kernel<false><<<kDualRoots, kThreads, 0, s>>>(nodes, num_nodes, bodies, (int) n, G, eps, theta, acc,
                                                        counts, ws.roots, ws.num_roots, ws.arena, (int) ws.arena_words,

@@ -32,3 +32,10 @@ def test_clustered(nb, oracle, n, leaf):
     pm, _ = two_spheres(nb, n, seed=n)
     pm[: n // 8] = pm[n // 8: 2 * (n // 8)]  # pairs of coincident bodies
     check_counts(nb, oracle, pm, leaf, 0.5)
+
+
+@pytest.mark.parametrize("n,leaf", [(131_071, 32), (131_072, 32), (131_072, 16), (160_001, 8)])
+def test_frontier_sizes(nb, oracle, n, leaf):
+    """Both sides of the line at which the frontier and the near-field units grow, and small leaves above it."""
+    pm, _ = two_spheres(nb, n, seed=4)
+    check_counts(nb, oracle, pm, leaf, 0.7)
