@@ -4,7 +4,7 @@
 // A block of eight warps stages 256 source bodies at a time in shared memory (coalesced float4 loads,
 // double buffered, one barrier per tile) and sweeps the tile with broadcast reads. Its targets:
 //   Z = 8: 32 targets (FP32: 64 where there are enough), every warp taking an eighth of each tile;
-//   Z = 1: 256 targets (FP32: 512), for target counts that fill the GPU that way already.
+//   Z = 1: 256 targets (FP32: 512), for target counts that fill the GPU that way already or few sources.
 // Up to eight blocks of a cluster share the sources of the same targets. Partial sums meet in shared
 // memory, warps first, then the cluster's blocks (distributed shared memory), in a fixed order.
 // One thread per target over all sources, 256 targets per block, left 30,011 targets on 118 of 148
@@ -341,10 +341,18 @@ void launch_clusters(void (*kernel)(Params...), int64_t target_blocks, int clust
     cudaLaunchKernelEx(&cfg, kernel, Params(args)...);
 }
 
-// From this many targets on, 256 per block fill the GPU for several waves, and sources are read from
-// L2 once per 256 targets instead of once per 32.
-constexpr int64_t kWideTargets = 300000;
-// From this many targets on, two per lane leave enough blocks.
+// The wide form (Z = 1) reads sources once per 256 or 512 targets instead of once per 32 or 64, but its blocks are
+// few and long: a wave that is begun costs a whole one. Where there are this many targets it pays, and, with few
+// sources, where the warps' partial sums would cost as much as the sum. Measured, us, Z = 8 / Z = 1:
+//   FP32, 32,768 sources: 150,000 targets 2144 / 2132, 304,000 4143 / 5023, 380,000 5159 / 5975, 450,000 6110 / 5969,
+//     800,000 10799 / 10732
+//   FP64, 4,096 sources: 310,000 1557 / 1690, 500,000 2490 / 2578, 700,000 3472 / 3467, 2 10^6 9884 / 9515
+//   100 sources, FP32: 100,000 11.7 / 11.8, 200,000 18.8 / 16.0, 10^6 71 / 50, FP64: 100,000 23.8 / 22.5, 200,000 40.6 / 37.0;
+//   300 sources, FP32: 100,000 20.1 / 25.9, 200,000 35.0 / 34.5
+constexpr int64_t kWideTargets32 = 440000, kWideTargets64 = 700000;
+bool wide_targets(int64_t targets, int64_t n, int64_t wide) { return targets >= (n <= 128 ? 100000 : wide); }
+// From this many targets on, two per lane leave enough blocks. FP32, us, T = 1 / T = 2: 4,096 sources: 4,096 targets 16.9 /
+// 17.3, 8,192 26.2 / 26.2, 20,000 53.1 / 48.7; 32,768 sources: 6,000 111 / 107, 8,192 147 / 139, 65,536 1039 / 942.
 constexpr int64_t kPairTargets = 8192;
 
 }  // namespace
@@ -366,7 +374,7 @@ void launch_direct_f32(const float4 *bodies, int64_t n, const float4 *targets, i
         launch_clusters(eps == 0.f ? narrow : soft, (nt + per_block - 1) / per_block, cluster, s, bodies, n, targets, nt, G,
                         eps, acc);
     };
-    if (shape_targets >= kWideTargets)
+    if (wide_targets(shape_targets, n, kWideTargets32))
         launch(direct_f32_kernel<true, 1, 2>, direct_f32_kernel<false, 1, 2>, 2 * kThreads, 1);
     else if (shape_targets >= kPairTargets)
         launch(direct_f32_kernel<true, 8, 2>, direct_f32_kernel<false, 8, 2>, 64, cluster_for((shape_targets + 63) / 64, n));
@@ -377,7 +385,7 @@ void launch_direct_f32(const float4 *bodies, int64_t n, const float4 *targets, i
 void launch_direct_f64(const float4 *bodies, int64_t n, const float4 *targets, int64_t nt, double G, double eps,
                        double *acc3, cudaStream_t s) {
     if (nt <= 0) return;
-    if (nt >= kWideTargets) {
+    if (wide_targets(nt, n, kWideTargets64)) {
         launch_clusters(direct_f64_kernel<1>, (nt + kThreads - 1) / kThreads, 1, s, bodies, n, targets, nt, G, eps, acc3);
     } else {
         const int64_t blocks = (nt + 31) / 32;

@@ -46,7 +46,7 @@ def test_wide_direct_sums(nb):
     import torch
 
     pm, _ = nb.scenarios.plummer(300, seed=3)
-    nt = 300_037  # one thread per target
+    nt = 300_037  # one warp in eight per tile; the wide forms: test_wide_lines
     t = torch.from_numpy(pm[np.arange(nt) % 300]).cuda()
     b = torch.from_numpy(pm).cuda()
     a32 = torch.zeros(nt, 4, device="cuda")
@@ -58,6 +58,28 @@ def test_wide_direct_sums(nb):
         s.direct_device(300, b.data_ptr(), nt, t.data_ptr(), a64.data_ptr(), 64)
         s.synchronize()
     at = np.arange(nt) % 300
+    assert (np.abs(a32.cpu().numpy()[:, :3] - ref[at]) <= 4e-6 * size[at]).all()
+    assert (np.abs(a64.cpu().numpy() - ref[at]) <= 2e-14 * size[at]).all()
+
+
+@pytest.mark.parametrize("n,nt", [(1, 100_000), (128, 100_003), (128, 99_999), (129, 300_000), (200, 700_001)])
+def test_wide_lines(nb, n, nt):
+    """Both sides of the lines of the wide form, by targets and by sources."""
+    import torch
+
+    pm, _ = nb.scenarios.plummer(max(n, 8), seed=n)
+    pm = pm[:n]
+    own = np.concatenate([pm, np.float32([[0.5, -0.25, 0.125, 0.0]])])
+    at = np.arange(nt) % len(own)
+    b, t = torch.from_numpy(pm).cuda(), torch.from_numpy(own[at]).cuda()
+    a32 = torch.zeros(nt, 4, device="cuda")
+    a64 = torch.zeros(nt, 3, device="cuda", dtype=torch.float64)
+    torch.cuda.synchronize()
+    ref, size = reference(pm, own, float(np.float32(1e-4)))
+    with nb.NaiveSolver(None, nb.Gravity(1.0, 1e-4)) as s:
+        s.direct_device(n, b.data_ptr(), nt, t.data_ptr(), a32.data_ptr(), 32)
+        s.direct_device(n, b.data_ptr(), nt, t.data_ptr(), a64.data_ptr(), 64)
+        s.synchronize()
     assert (np.abs(a32.cpu().numpy()[:, :3] - ref[at]) <= 4e-6 * size[at]).all()
     assert (np.abs(a64.cpu().numpy() - ref[at]) <= 2e-14 * size[at]).all()
 
