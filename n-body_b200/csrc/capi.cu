@@ -395,7 +395,8 @@ int dual_traverse(nb_ctx *ctx, int64_t n, int64_t first, int64_t count, cudaStre
     NearPool &np = ctx->dws.near;
     for (int attempt = 0;; ++attempt) {
         launch_dual_traverse(ctx->dnodes, ctx->tw.num_nodes, ctx->pos, n, ctx->cfg.G, ctx->cfg.epsilon,
-                             ctx->cfg.theta, ctx->cfg.max_leaf_size, ctx->acc, ctx->counts, ctx->dws, ctx->err, s, first, first + count);
+                             ctx->cfg.theta, ctx->cfg.max_leaf_size, ctx->acc, ctx->counts, ctx->dws, ctx->err, s,
+                             first, first + count);
         unsigned long long *h = ctx->host_scratch;
         SpillPool &sp = ctx->dws.spill;
         NB_TRY(cudaMemcpyAsync(h, np.counters, 4 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s),
@@ -1099,7 +1100,6 @@ static int build_batch_tables(nb_ctx *ctx, int32_t count, const int64_t *sizes, 
     const int64_t largest = count > 0 ? *std::max_element(sizes, sizes + count) : 1;
     ctx->inst_bbox_slices = (int) std::min<int64_t>(std::max<int64_t>((largest + 8191) / 8192, 1), 64);
     const int passes = count > 256 ? 2 : 1;
-    const int64_t tiles = sort_tiles(n);
     if (n > ctx->batch_body_cap) {  // per-body buffers grow only
         dev_free(ctx->inst_of); dev_free(ctx->ikeys); dev_free(ctx->ikeys2); dev_free(ctx->ivals);
         dev_free(ctx->ivals2); dev_free(ctx->inst_lookback);
@@ -1133,7 +1133,6 @@ static int build_batch_tables(nb_ctx *ctx, int32_t count, const int64_t *sizes, 
     }
     if (!ctx->inst_hist) NB_TRY(dev_alloc(&ctx->inst_hist, hist.size()), "alloc batch");
     if (!ctx->inst_tiles) NB_TRY(dev_alloc(&ctx->inst_tiles, 8), "alloc batch");
-    (void) tiles;
     int *group_first_dev = ctx->group_first;
     cudaStream_t s = ctx->stream;
     NB_TRY(cudaMemcpyAsync(ctx->inst_theta2, theta2.data(), theta2.size() * sizeof(float), cudaMemcpyHostToDevice, s),

@@ -1015,7 +1015,7 @@ __global__ void __launch_bounds__(512) load_balanced_break_kernel(DualNodes node
         if (tid == 0) break_by_heap(nodes, nn, S.size, S.id, roots, num_roots, err);
         return;
     }
-    // starting nodes: not split, below a split one (or the root); listed in the parent array's place
+    // starting nodes: not split, below a split one (or the root); listed in place of the right children
     for (int i = tid; i < count; i += blockDim.x)
         if (S.split[i] != 2 && (i == 0 || S.split[S.parent[i]] == 2)) S.right[atomicAdd(&s_roots, 1)] = i;
     __syncthreads();
@@ -1570,7 +1570,8 @@ __global__ void __launch_bounds__(kNearThreads, 8) near_kernel(DualNodes nodes, 
 
 // Passive nodes of at most this many bodies below a larger parent are handed to the second kernel, which balances
 // them over the whole GPU: 64 bodies in small sets (more would leave the first kernel's tasks too large),
-// sqrt(n) / 2 above (fewer nodes, longer lists each), less for leaves below 64, whose deeper subtrees cost more. Whole traversal, ms, 64 / 128 / 181 / 256:
+// sqrt(n) / 2 above (fewer nodes, longer lists each), less for leaves below 64, whose deeper subtrees cost
+// more. Whole traversal, ms, frontier 64 / 128 / 181 / 256:
 //   leaf 8  theta 0.6  131,072: 20.7 (64) / 23.6 (181), 250,000: 51.0 (64) / 51.8 (250)
 //   leaf 16 theta 0.6  131,072:  9.4 /  9.6 / 10.4 / 11.6, 180,000: 14.6 / 14.1 / 14.3 / 15.3, 250,000: 22.8 / 21.4 / 21.2 / 21.8
 //   leaf 32 theta 0.5   90,000:  4.9 /  4.8 /  5.4 /  6.2, 131,072:  7.1 /  6.8 /  7.2 /  8.0, 250,000: 17.7 / 15.5 / 15.2 / 15.3

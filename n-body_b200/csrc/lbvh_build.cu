@@ -836,8 +836,9 @@ __global__ void __launch_bounds__(kClimbThreads) summarize_kernel(const float4 *
 // and a block's 128 threads take its leaf parents in turn. So the size grows with n, such that some 400 blocks or
 // more are left (twice as large for the octupole, whose records above the blocks cost more), up to a
 // number of leaf parents that keeps the threads busy. A set that one block holds, with a leaf parent or two per
-// thread, takes one block, and two or three blocks of 1024 where that is as fast (2,000 bodies of two spheres, octupole, leaf
-// 16: 365 us a pass with 1024, 393 with 128). Whole build, us, 128 / 256 / 512 / 1024 / 2048 / 4096 nodes per block, quadrupole unless stated:
+// thread, takes one block, and two or three blocks of 1024 where that is as fast (2,000 bodies of two spheres,
+// octupole, leaf 16: 365 us a pass with 1024, 393 with 128). Whole build, us, 128 / 256 / 512 / 1024 / 2048 / 4096
+// nodes per block, quadrupole unless stated:
 //   1,000 bodies    leaf 2   73 / 73 / 82 / 83 / 81 / 84, leaf 16 65 / 65 / 65 / 47 / 47 / 47
 //   3,000           leaf 16  79 / 77 / 77 / 79 / 78 / 85, leaf 32 75 / - / - / 79 / 77 / 62
 //   20,000          leaf 1   114 / 130 / 145 / 172 / 280 / 483, leaf 16 106 / 107 / 112 / 111 / 122 / 148

@@ -115,16 +115,13 @@ __device__ __forceinline__ float ref_dist2(float px, float py, float pz, float4 
     return fadd(fadd(fmul(dx, dx), fmul(dy, dy)), fmul(dz, dz));
 }
 
-// on = false makes the term exactly zero (a select, not a branch, so that lanes whose target does
-// not take the term run the same instructions).
 template<bool EPS0>
-__device__ __forceinline__ void pair_term(float4 p, float4 b, float eps, float &ax, float &ay, float &az,
-                                          bool on = true) {
+__device__ __forceinline__ void pair_term(float4 p, float4 b, float eps, float &ax, float &ay, float &az) {
     const float rx = p.x - b.x, ry = p.y - b.y, rz = p.z - b.z;
     const float r2 = fmaf(rx, rx, fmaf(ry, ry, fmaf(rz, rz, eps)));
     if (EPS0 && r2 == 0.f) return;  // equal positions contribute nothing (Gravity.h:203)
     const float inv = rsqrt_hw(r2);
-    const float s = on ? b.w * (inv * inv * inv) : 0.f;
+    const float s = b.w * (inv * inv * inv);
     ax = fmaf(-rx, s, ax);
     ay = fmaf(-ry, s, ay);
     az = fmaf(-rz, s, az);
