@@ -216,7 +216,7 @@ __global__ void __launch_bounds__(kThreads) direct_f64_kernel(const float4 *__re
 // pair of tiles is evaluated once: tile I takes the tiles I + 0 .. I + tiles / 2 around the ring of
 // tiles (the farthest only from the lower half when the tile count is even), block y of its row an
 // equal share of them. parts[2 block + {0, 1}] = (kinetic, sum over ordered pairs), in a fixed order.
-// Bound by the FP64 pipe: 13 operations per unordered pair. 40,009 bodies: 8.93 ms before, 0.77 ms now.
+// Bound by the FP64 pipe: 13 operations per unordered pair. 40,009 bodies: 8.93 ms before, 0.74 ms now.
 __global__ void __launch_bounds__(kThreads) energy_f64_kernel(const float4 *__restrict__ bodies,
                                                               const float4 *__restrict__ vel, int64_t n, double eps,
                                                               int tiles, double *__restrict__ parts) {
