@@ -40,7 +40,6 @@
 #include <algorithm>
 #include <cfloat>
 #include <climits>
-#include <cmath>
 #include <memory>
 #include <new>
 
@@ -1026,12 +1025,13 @@ int resident_warps(int device) {
 // group. The team form has one walking warp in eight and four blocks per SM, so it loses where the groups alone
 // fill the GPU. The line, in groups per SM:
 //   - one wave of teams (four) always gains;
-//   - above, larger leaves shift work from the walk to the leaf warps, and the line with it; theta above 0.5
-//     opens fewer leaves (the exponent fits theta 0.7 and 1);
+//   - above, larger leaves shift work from the walk to the leaf warps, and the line with it; a larger theta opens
+//     fewer leaves, from 0.5 on at small ones, from 0.6 on at leaves of 64 (a straight line down to a fifth at theta 1);
 //   - a slice of a larger set (a shard) has no sparse outskirts, whose few long groups hold one warp up
 //     longest, and a deeper tree to walk;
 //   - trees of few leaves give a group hardly more to do than a team's start and end cost.
-// Measured, time with one warp over time with teams (g: groups per SM):
+// Measured, time with one warp over time with teams (g: groups per SM; Plummer spheres keep teams worth while to larger
+// sets than balls, the line lies between):
 //   whole sets at theta 0.5, Plummer and ball: leaf 1 1.07-1.09 at g 6, 0.96-1.07 at 8; leaf 8 1.02-1.15 at 10,
 //     0.83-0.87 at 14; leaf 16 1.03-1.10 at 14, 0.96-0.99 at 18; leaf 32 0.98-1.10 at 30; leaf 64 0.99-1.07 at 54;
 //   theta 0.7: leaf 8 1.00-1.08 at 10, 0.90-0.96 at 12; leaf 16 1.07-1.14 at 12, 0.95 at 14; leaf 32 1.04-1.18
@@ -1045,8 +1045,8 @@ int resident_warps(int device) {
 // at theta 0.5 and up to 50 groups per SM, 1.04-1.7 for leaves of 1000).
 int64_t team_groups(int device, int leaf, float theta, int64_t tree_bodies, bool slice) {
     if (leaf > 64) return 0;
-    const double opened = theta > 0.5f ? std::pow(0.5 / theta, 1.75) : 1.0;
-    const double most = 6.0 + 0.75 * leaf * opened * (slice ? 0.45 : 1.0);
+    const double opened = std::min(1.0, std::max(0.2, 1.0 - 2.5 * (theta - (0.5 + leaf / 640.0))));
+    const double most = 6.0 + 0.75 * (leaf * opened * (slice ? 0.45 : 1.0) + 1.5 * (1.0 - opened));
     const double few = std::min(1.0, (double) tree_bodies / (128.0 * leaf));
     return (int64_t) (sm_count(device) * (4.0 + (most - 4.0) * few * few));
 }
